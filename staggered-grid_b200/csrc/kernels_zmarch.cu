@@ -42,8 +42,9 @@
 // The source (dt*dt*s(it) on txx, tyy, tzz, OPT/ElasticWaveEquation.cu:206-221)
 // is applied to the staged copies the velocity update reads and to the old
 // value the stress update accumulates onto, which reproduces the reference's
-// store-then-read order exactly; receivers are written from registers (with
-// 16-bit storage both run as the 16-bit family's own kernels).
+// store-then-read order exactly; receivers are recorded by the whole CTA after
+// their plane's block barrier (record_plane; with 16-bit storage both run as
+// the 16-bit family's own kernels).
 // Arithmetic per cell is the same sequence as kernels_simple.cu and the oracle.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -310,17 +311,14 @@ __device__ __forceinline__ bool vel_item(const ZMaps &mp, const Model &m, const 
         }
     }
 
-    // receivers of this tile, sorted by z: skip those below the chunk
-    int rp = H ? 0 : g.rec_off[tile];
-    const int rend = H ? 0 : g.rec_off[tile + 1];
-    while (rp < rend && g.rec_list[rp].z < gz0) ++rp;
-    int rz = rp < rend ? g.rec_list[rp].z : 0x7fffffff;   // z of the next receiver
+    RecCursor rec{0, 0, 0, 0x7fffffff};   // receivers at or above the chunk
+    if constexpr (!H) rec = rec_seek(g, tile, gz0);
 
     bool failed = false, abort = false;
     int cz = t.zs;
     const bool src_near = !H && sr.src >= 0 && sy >= t.gy0 - 5 && sy < t.gy0 + TY + 5 && sx >= t.gx0 - 8 &&
                           sx < t.gx0 + TX + 8;
-    // One plane.  GEN selects the general path (PML cells, source, receivers);
+    // One plane.  GEN selects the general path (PML cells, source);
     // the interior-only path is used for every other tile-plane.  Returns
     // false when the block votes to abort.
     auto plane = [&](auto gen_tag) -> bool {
@@ -521,21 +519,7 @@ __device__ __forceinline__ bool vel_item(const ZMaps &mp, const Model &m, const 
             put(fld(0) + ci, 0, vnew[0]);
             put(fld(1) + ci, 1, vnew[1]);
             put(fld(2) + ci, 2, vnew[2]);
-            // receivers of velocity components at this cell (list sorted by z)
-            if (GEN && !H && gz == rz && it >= 0 && it < sr.nt) {
-                for (int r = rp; r < rend && g.rec_list[r].z == gz; ++r) {
-                    const int4 q = g.rec_list[r];
-                    if (q.x == gx && q.y == gyc[c] && q.w <= 2)
-                        sr.traces[(int64_t)it * sr.nrec + g.rec_idx[r]] =
-                            q.w == 0 ? vnew[0] : q.w == 1 ? vnew[1] : vnew[2];
-                }
-            }
         }
-        if (GEN && gz == rz) {
-            while (rp < rend && g.rec_list[rp].z == gz) ++rp;
-            rz = rp < rend ? g.rec_list[rp].z : 0x7fffffff;
-        }
-
         // every thread is done with this stage: vote on aborts, then refill it
         if (__syncthreads_or(failed)) return false;
         if (cz + S < t.ze) {
@@ -544,6 +528,9 @@ __device__ __forceinline__ bool vel_item(const ZMaps &mp, const Model &m, const 
                 vel_issue<TY, ES>(mybox, nbox, st, &bar[s], cz + S, warp);
             }
             issued_end = cz + S + 1;
+        }
+        if constexpr (!H) {
+            if (gz == rec.z) record_plane(m, g, sr, it, true, rec);
         }
         if (MANY) pbits ^= 1u << s;
         if (++stage == S) {
@@ -554,7 +541,7 @@ __device__ __forceinline__ bool vel_item(const ZMaps &mp, const Model &m, const 
     };
     for (; cz < t.ze; ++cz) {
         const int gzp = cz + kHalo;
-        const bool gen = t.xy_pml || bandz(m, gzp) != 0 || (src_near && (gzp == sz || gzp + 5 == sz)) || gzp == rz;
+        const bool gen = t.xy_pml || bandz(m, gzp) != 0 || (src_near && (gzp == sz || gzp + 5 == sz));
         if (!(gen ? plane(std::true_type{}) : plane(std::false_type{}))) {
             abort = true;
             break;
@@ -711,10 +698,8 @@ __device__ __forceinline__ bool str_item(const ZMaps &mp, const Model &m, const 
         }
     }
 
-    int rp = H ? 0 : g.rec_off[tile];
-    const int rend = H ? 0 : g.rec_off[tile + 1];
-    while (rp < rend && g.rec_list[rp].z < gz0) ++rp;
-    int rz = rp < rend ? g.rec_list[rp].z : 0x7fffffff;
+    RecCursor rec{0, 0, 0, 0x7fffffff};   // receivers at or above the chunk
+    if constexpr (!H) rec = rec_seek(g, tile, gz0);
 
     bool failed = false, abort = false;
     int cz = t.zs;
@@ -905,21 +890,7 @@ __device__ __forceinline__ bool str_item(const ZMaps &mp, const Model &m, const 
                 }
                 put(fld(3 + q) + ci, 3 + q, snew[q]);
             }
-            if (GEN && !H && gz == rz && it >= 0 && it < sr.nt) {
-                for (int r = rp; r < rend && g.rec_list[r].z == gz; ++r) {
-                    const int4 q = g.rec_list[r];
-                    if (q.x == gx && q.y == gyc[c] && q.w >= 3)
-                        sr.traces[(int64_t)it * sr.nrec + g.rec_idx[r]] =
-                            q.w == 3 ? snew[0] : q.w == 4 ? snew[1] : q.w == 5 ? snew[2]
-                          : q.w == 6 ? snew[3] : q.w == 7 ? snew[4] : snew[5];
-                }
-            }
         }
-        if (GEN && gz == rz) {
-            while (rp < rend && g.rec_list[rp].z == gz) ++rp;
-            rz = rp < rend ? g.rec_list[rp].z : 0x7fffffff;
-        }
-
         if (__syncthreads_or(failed)) return false;
         if (cz + S < t.ze) {
             if (lx == 0) {
@@ -927,6 +898,9 @@ __device__ __forceinline__ bool str_item(const ZMaps &mp, const Model &m, const 
                 str_issue<TY, ES>(mybox, nbox, st, &bar[s], cz + S, warp);
             }
             issued_end = cz + S + 1;
+        }
+        if constexpr (!H) {
+            if (gz == rec.z) record_plane(m, g, sr, it, false, rec);
         }
         if (MANY) pbits ^= 1u << s;
         if (++stage == S) {
@@ -937,7 +911,7 @@ __device__ __forceinline__ bool str_item(const ZMaps &mp, const Model &m, const 
     };
     auto run = [&](auto p_tag) -> bool {
         const int gzp = cz + kHalo;
-        const bool gen = t.xy_pml || bandz(m, gzp) != 0 || gzp == sz || gzp == rz;
+        const bool gen = t.xy_pml || bandz(m, gzp) != 0 || gzp == sz;
         prefetch(cz + 1);
         return gen ? plane(std::true_type{}, p_tag) : plane(std::false_type{}, p_tag);
     };

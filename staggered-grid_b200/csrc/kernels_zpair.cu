@@ -19,7 +19,7 @@
 // loads; z differences on FP32x2 from register queues of float2.  Each lane
 // of a packed operation rounds exactly as the scalar operation, so results
 // are bit-identical to kernels_zmarch.cu, kernels_simple.cu and the oracle.
-// Tile-planes with PML cells, the source or receivers take the general path,
+// Tile-planes with PML cells or the source take the general path,
 // which updates cell by cell; every other tile-plane updates the pair on
 // FP32x2 and stores it with one 8-byte store per field.
 #include <cuda.h>
@@ -398,17 +398,14 @@ __device__ __forceinline__ bool vel_pair(const VelMaps &mp, const Model &m, cons
         qzz[k] = zz;
     }
 
-    // receivers of this tile, sorted by z: skip those below the chunk
-    int rp = H ? 0 : g.rec_off[tile];
-    const int rend = H ? 0 : g.rec_off[tile + 1];
-    while (rp < rend && g.rec_list[rp].z < gz0) ++rp;
-    int rz = rp < rend ? g.rec_list[rp].z : 0x7fffffff;
+    RecCursor rec{0, 0, 0, 0x7fffffff};   // receivers at or above the chunk
+    if constexpr (!H) rec = rec_seek(g, tile, gz0);
 
     bool failed = false, abort = false;
     int cz = t.zs;
     const bool src_near = !H && sr.src >= 0 && sy >= t.gy0 - 5 && sy < t.gy0 + PY + 5 && sx >= t.gx0 - 8 &&
                           sx < t.gx0 + PX + 8;
-    // One plane.  GEN selects the general path (PML cells, source, receivers);
+    // One plane.  GEN selects the general path (PML cells, source);
     // every other tile-plane takes the packed interior path.  ODD: the second
     // plane of a pair (queue window one entry further).  Returns false when
     // the block votes to abort.
@@ -504,16 +501,6 @@ __device__ __forceinline__ bool vel_pair(const VelMaps &mp, const Model &m, cons
                     note_max16s(smax, 1, fmaxf(fabsf(v1.x), pc.act1 ? fabsf(v1.y) : 0.0f));
                     note_max16s(smax, 2, fmaxf(fabsf(v2.x), pc.act1 ? fabsf(v2.y) : 0.0f));
                 }
-                if (!H && GEN && gz == rz && it >= 0 && it < sr.nt) {
-                    for (int r = rp; r < rend && g.rec_list[r].z == gz; ++r) {
-                        const int4 q = g.rec_list[r];
-                        if (q.y == pc.gy && q.w <= 2 && (q.x == pc.gx || (pc.act1 && q.x == pc.gx + 1))) {
-                            const int c = q.x - pc.gx;
-                            sr.traces[(int64_t)it * sr.nrec + g.rec_idx[r]] =
-                                q.w == 0 ? lane_of(v0, c) : q.w == 1 ? lane_of(v1, c) : lane_of(v2, c);
-                        }
-                    }
-                }
             } else {
                 // general path, cell by cell; PML cells through their split fields
 #pragma unroll
@@ -575,20 +562,8 @@ __device__ __forceinline__ bool vel_pair(const VelMaps &mp, const Model &m, cons
                         if (track) note_max16s(smax, q, vnew[q]);
                         SA::put1(F.f(q) + cc, vnew[q], F.inv(q));
                     }
-                    if (!H && gz == rz && it >= 0 && it < sr.nt) {
-                        for (int r = rp; r < rend && g.rec_list[r].z == gz; ++r) {
-                            const int4 q = g.rec_list[r];
-                            if (q.x == pc.gx + c && q.y == pc.gy && q.w <= 2)
-                                sr.traces[(int64_t)it * sr.nrec + g.rec_idx[r]] =
-                                    q.w == 0 ? vnew[0] : q.w == 1 ? vnew[1] : vnew[2];
-                        }
-                    }
                 }
             }
-        }
-        if (GEN && gz == rz) {
-            while (rp < rend && g.rec_list[rp].z == gz) ++rp;
-            rz = rp < rend ? g.rec_list[rp].z : 0x7fffffff;
         }
         if constexpr (Q == 1) {   // after a pair of planes the queues move by two
 #pragma unroll
@@ -608,6 +583,9 @@ __device__ __forceinline__ bool vel_pair(const VelMaps &mp, const Model &m, cons
             }
             issued_end = cz + S + 1;
         }
+        if constexpr (!H) {
+            if (gz == rec.z) record_plane(m, g, sr, it, true, rec);
+        }
         if (++stage == S) stage = 0;
         return true;
     };
@@ -615,8 +593,7 @@ __device__ __forceinline__ bool vel_pair(const VelMaps &mp, const Model &m, cons
     using T0 = std::false_type;
     for (; cz < t.ze; ++cz) {
         const int gzp = cz + kHalo;
-        const bool gen = t.xy_pml || bandz(m, gzp) != 0 || (src_near && (gzp == sz || gzp + 5 == sz)) ||
-                         gzp == rz;
+        const bool gen = t.xy_pml || bandz(m, gzp) != 0 || (src_near && (gzp == sz || gzp + 5 == sz));
         const bool odd = ((cz - t.zs) & 1) != 0;
         const bool ok = odd ? (gen ? plane(T1{}, T1{}) : plane(T0{}, T1{})) : (gen ? plane(T1{}, T0{}) : plane(T0{}, T0{}));
         if (!ok) {
@@ -705,10 +682,8 @@ __device__ __forceinline__ bool str_pair(const StrMaps &mp, const Model &m, cons
         qz[k] = SA::pair(F.f(2) + pc.col + (uint32_t)(gz0 - 5 + k) * PL, bcast(F.sc(2)));
     }
 
-    int rp = H ? 0 : g.rec_off[tile];
-    const int rend = H ? 0 : g.rec_off[tile + 1];
-    while (rp < rend && g.rec_list[rp].z < gz0) ++rp;
-    int rz = rp < rend ? g.rec_list[rp].z : 0x7fffffff;
+    RecCursor rec{0, 0, 0, 0x7fffffff};   // receivers at or above the chunk
+    if constexpr (!H) rec = rec_seek(g, tile, gz0);
 
     bool failed = false, abort = false;
     int cz = t.zs;
@@ -780,13 +755,6 @@ __device__ __forceinline__ bool str_pair(const StrMaps &mp, const Model &m, cons
                 for (int q = 0; q < 6; ++q) {
                     SA::put2(F.f(3 + q) + ci, sn[q], bcast(F.inv(3 + q)), pc.act1);
                     if (track) note_max16s(smax, 3 + q, fmaxf(fabsf(sn[q].x), pc.act1 ? fabsf(sn[q].y) : 0.0f));
-                }
-                if (!H && GEN && gz == rz && it >= 0 && it < sr.nt) {
-                    for (int r = rp; r < rend && g.rec_list[r].z == gz; ++r) {
-                        const int4 q = g.rec_list[r];
-                        if (q.y == pc.gy && q.w >= 3 && (q.x == pc.gx || (pc.act1 && q.x == pc.gx + 1)))
-                            sr.traces[(int64_t)it * sr.nrec + g.rec_idx[r]] = lane_of(pick6(sn, q.w - 3), q.x - pc.gx);
-                    }
                 }
             } else {
 #pragma unroll
@@ -870,19 +838,8 @@ __device__ __forceinline__ bool str_pair(const StrMaps &mp, const Model &m, cons
                         if (track) note_max16s(smax, 3 + q, snew[q]);
                         SA::put1(F.f(3 + q) + cc, snew[q], F.inv(3 + q));
                     }
-                    if (!H && gz == rz && it >= 0 && it < sr.nt) {
-                        for (int r = rp; r < rend && g.rec_list[r].z == gz; ++r) {
-                            const int4 q = g.rec_list[r];
-                            if (q.x == pc.gx + c && q.y == pc.gy && q.w >= 3)
-                                sr.traces[(int64_t)it * sr.nrec + g.rec_idx[r]] = pick6(snew, q.w - 3);
-                        }
-                    }
                 }
             }
-        }
-        if (GEN && gz == rz) {
-            while (rp < rend && g.rec_list[rp].z == gz) ++rp;
-            rz = rp < rend ? g.rec_list[rp].z : 0x7fffffff;
         }
         if constexpr (Q == 1) {
 #pragma unroll
@@ -901,6 +858,9 @@ __device__ __forceinline__ bool str_pair(const StrMaps &mp, const Model &m, cons
             }
             issued_end = cz + S + 1;
         }
+        if constexpr (!H) {
+            if (gz == rec.z) record_plane(m, g, sr, it, false, rec);
+        }
         if (++stage == S) stage = 0;
         return true;
     };
@@ -908,7 +868,7 @@ __device__ __forceinline__ bool str_pair(const StrMaps &mp, const Model &m, cons
     using T0 = std::false_type;
     for (; cz < t.ze; ++cz) {
         const int gzp = cz + kHalo;
-        const bool gen = t.xy_pml || bandz(m, gzp) != 0 || gzp == sz || gzp == rz;
+        const bool gen = t.xy_pml || bandz(m, gzp) != 0 || gzp == sz;
         const bool odd = ((cz - t.zs) & 1) != 0;
         const bool ok = odd ? (gen ? plane(T1{}, T1{}) : plane(T0{}, T1{})) : (gen ? plane(T1{}, T0{}) : plane(T0{}, T0{}));
         if (!ok) {

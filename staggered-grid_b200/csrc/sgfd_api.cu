@@ -333,30 +333,33 @@ int upload_zrec(sgfd_solver *h, const std::vector<int4> &rec) {
     }
     std::vector<int> off(tiles + 1, 0);
     std::vector<int4> list;
-    std::vector<int> idx;
+    std::vector<int2> col;
     for (int t = 0; t < tiles; ++t) {
         auto &b = buckets[t];
         std::stable_sort(b.begin(), b.end(), [](const std::pair<int4, int> &a, const std::pair<int4, int> &c) {
             return a.first.z < c.first.z;
         });
-        for (auto &e : b) { list.push_back(e.first); idx.push_back(e.second); }
+        const int first = (int)list.size();
+        for (auto &e : b) { list.push_back(e.first); col.push_back(make_int2(e.second, 0)); }
         off[t + 1] = (int)list.size();
+        for (int i = (int)list.size() - 1; i >= first; --i)   // end of the entries on the entry's plane
+            col[i].y = i + 1 < off[t + 1] && list[i + 1].z == list[i].z ? col[i + 1].y : i + 1;
     }
-    cudaFree(h->zrec_off); cudaFree(h->zrec_list); cudaFree(h->zrec_idx);
-    h->zrec_off = nullptr; h->zrec_list = nullptr; h->zrec_idx = nullptr;
+    cudaFree(h->zrec_off); cudaFree(h->zrec_list); cudaFree(h->zrec_col);
+    h->zrec_off = nullptr; h->zrec_list = nullptr; h->zrec_col = nullptr;
     const size_t nl = std::max<size_t>(list.size(), 1);
     cudaError_t e = dev_malloc(h, &h->zrec_off, off.size() * sizeof(int));
     if (e == cudaSuccess) e = dev_malloc(h, &h->zrec_list, nl * sizeof(int4));
-    if (e == cudaSuccess) e = dev_malloc(h, &h->zrec_idx, nl * sizeof(int));
+    if (e == cudaSuccess) e = dev_malloc(h, &h->zrec_col, nl * sizeof(int2));
     if (e != cudaSuccess) { cudaGetLastError(); return fail(h, SGFD_ERR_ALLOC, "receiver lists"); }
     SG_CUDA(h, cudaMemcpy(h->zrec_off, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice), "receiver lists");
     if (!list.empty()) {
         SG_CUDA(h, cudaMemcpy(h->zrec_list, list.data(), list.size() * sizeof(int4), cudaMemcpyHostToDevice), "receiver lists");
-        SG_CUDA(h, cudaMemcpy(h->zrec_idx, idx.data(), idx.size() * sizeof(int), cudaMemcpyHostToDevice), "receiver lists");
+        SG_CUDA(h, cudaMemcpy(h->zrec_col, col.data(), col.size() * sizeof(int2), cudaMemcpyHostToDevice), "receiver lists");
     }
     h->zg.rec_off = h->zrec_off;
     h->zg.rec_list = h->zrec_list;
-    h->zg.rec_idx = h->zrec_idx;
+    h->zg.rec_col = h->zrec_col;
     return SGFD_OK;
 }
 
@@ -569,7 +572,7 @@ void sgfd_destroy(sgfd_solver *h) {
     cudaFree(h->wavelet);
     cudaFree(h->zrec_off);
     cudaFree(h->zrec_list);
-    cudaFree(h->zrec_idx);
+    cudaFree(h->zrec_col);
     cudaFree(h->dev_err);
     cudaFree(h->h16_pool);
     cudaFree(h->hstate);

@@ -70,7 +70,7 @@ struct sgfd_solver {
     std::vector<int4> rec_host;   // receivers, for re-bucketing when the tiling changes
     int *zrec_off = nullptr;
     int4 *zrec_list = nullptr;
-    int *zrec_idx = nullptr;
+    int2 *zrec_col = nullptr;
     int *dev_err = nullptr;
     // CUDA-graph replay of sgfd_run
     cudaStream_t cap_stream = nullptr;
