@@ -195,6 +195,20 @@ __global__ void k_shear_means(Model m, int quirks, float *mxy, float *mxz, float
     myz[c] = hmean<FAST>(r[c], r[c + Y], r[c + Z], r[c + Y + Z]);
 }
 
+// The wave speed the damping of a PML cell scales with (damp_speed), from the
+// cell's own medium: the z-marching updates then load one value per PML cell
+// and step instead of mu, lambda and a square root.
+__global__ void k_damp_speed(Model m, Physics ph, float *vd) {
+    const int cx = blockIdx.x * kBX + threadIdx.x;
+    const int cy = blockIdx.y * kBY + threadIdx.y;
+    const int cz = blockIdx.z;
+    if (cx >= m.nxc || cy >= m.nyc) return;
+    const int x = cx + kHalo, y = cy + kHalo, z = cz + kHalo;
+    if (!(band(x, m.nx, m.pml) | band(y, m.ny, m.pml) | bandz(m, z))) return;
+    const int64_t c = pidx(m, x, y, z);
+    vd[pml_index(m, cx, cy, cz)] = damp_speed(ph, m.mu[c], m.b[c], m.lam[c]);
+}
+
 // Device step counter of a replayed CUDA graph: set before the first replay,
 // advanced by the last node of each replay.
 __global__ void k_counter(int *ctr, int value, int add) {
@@ -262,6 +276,14 @@ cudaError_t launch_shear_means(const Model &m, const Physics &ph, float *mxy, fl
     const dim3 grid((m.nxc + kBX - 1) / kBX, (m.nyc + kBY - 1) / kBY, m.nzc);
     if (ph.fast) k_shear_means<true><<<grid, block, 0, s>>>(m, ph.quirks, mxy, mxz, myz);
     else k_shear_means<false><<<grid, block, 0, s>>>(m, ph.quirks, mxy, mxz, myz);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_damp_speed(const Model &m, const Physics &ph, float *vd, cudaStream_t s) {
+    if (m.npml == 0) return cudaSuccess;
+    const dim3 block(kBX, kBY);
+    const dim3 grid((m.nxc + kBX - 1) / kBX, (m.nyc + kBY - 1) / kBY, m.nzc);
+    k_damp_speed<<<grid, block, 0, s>>>(m, ph, vd);
     return cudaGetLastError();
 }
 

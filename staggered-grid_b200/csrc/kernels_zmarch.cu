@@ -26,8 +26,12 @@
 //     registers before the plane's TMA wait; the stress update, which needs
 //     15 of them, loads them where they are used, so that it fits the 80
 //     registers per thread of three resident CTAs per SM, and brings them
-//     (and the buoyancy of the damping) into L2 one plane ahead: one bulk
-//     prefetch of the 15 stress rows per 32-cell split block.
+//     into L2 one plane ahead: one bulk prefetch of the 15 stress rows per
+//     32-cell split block.  The damping's wave speed is one value per PML
+//     cell, computed at the medium upload (Model::vd): 4 bytes per cell and
+//     update in place of mu and lambda (velocity) or the buoyancy (stress)
+//     and a square root.  150^3 grid with a 20-cell border 0.2298 to 0.2218
+//     ms/step, 394^3 2.579 to 2.542 ms/step.
 //   * 16-bit wavefield storage (ST = BF16 / F16, 32 x 8 tiles): the field
 //     boxes arrive as 16-bit values and are widened once per plane into an
 //     FP32 work buffer (float(h) * 2^e) before the same FP32 arithmetic.
@@ -330,19 +334,17 @@ __device__ __forceinline__ bool vel_item(const ZMaps &mp, const Model &m, const 
         const bool plane_pml = GEN && (t.xy_pml || kz != 0);
 
 
-        // PML cells: splits and the medium of the damping, loaded before the
-        // stage wait so that their latency overlaps the wait and the stencil
-        float opre[CELLS][9], mupre[CELLS], lampre[CELLS];
+        // PML cells: splits and damping speed, loaded before the stage wait so that their latency overlaps the wait and the stencil
+        float opre[CELLS][9], vpre[CELLS];
         if (plane_pml) {
 #pragma unroll
             for (int c = 0; c < CELLS; ++c) {
                 if (act[c] && (kx | kyc[c] | kz)) {
-                    const uint32_t ci = col[c] + (uint32_t)gz * PL;
-                    const auto *sp = spl() + split_base32(pml_plane_index(m, pcol[c], cz));
+                    const uint32_t pi = pml_plane_index(m, pcol[c], cz);
+                    const auto *sp = spl() + split_base32(pi);
 #pragma unroll
                     for (int q = 0; q < 9; ++q) opre[c][q] = ld(sp + q * kSplitBlock, q / 3);   // split q: field q / 3
-                    mupre[c] = m.mu[ci];
-                    lampre[c] = ph.damping == 1 ? m.lam[ci] : 0.f;
+                    vpre[c] = m.vd[pi];
                 }
             }
         }
@@ -475,7 +477,7 @@ __device__ __forceinline__ bool vel_item(const ZMaps &mp, const Model &m, const 
                 float mx = 1.f, my = 1.f, mz = 1.f;
         PDiv<FAST> px = 1, py = 1, pz = 1;
                 {
-                    const float v = damp_speed(ph, mupre[c], b0, lampre[c]);
+                    const float v = vpre[c];
                     if (kx) damp_factors<FAST>(ph, 0, ph.dx, kx, m.pml, v, mx, px);
                     if (ky) damp_factors<FAST>(ph, 1, ph.dy, ky, m.pml, v, my, py);
                     if (kz) damp_factors<FAST>(ph, 2, ph.dz, kz, m.pml, v, mz, pz);
@@ -705,8 +707,8 @@ __device__ __forceinline__ bool str_item(const ZMaps &mp, const Model &m, const 
     int cz = t.zs;
     int sz = -1;
     if (src >= 0) sz = (int)(src / m.plane);
-    // The PML cells' splits and buoyancy, loaded by plain loads after the
-    // stencil, are brought into L2 one plane ahead, while the plane before
+    // The PML cells' splits, loaded by plain loads after the stencil, are
+    // brought into L2 one plane ahead, while the plane before
     // them is computed (32 x 8 tiles: a warp's cells are one row): their
     // loads then wait on L2 rather than on HBM.  Two and three planes ahead
     // measured slower.
@@ -716,8 +718,7 @@ __device__ __forceinline__ bool str_item(const ZMaps &mp, const Model &m, const 
             const int kzp = bandz(m, pz + kHalo);
             if (!t.xy_pml && kzp == 0) return;
             const bool p = act[0] && (kx | kyc[0] | kzp);
-            if (prefetch_split_rows(spl(), p, pml_plane_index(m, pcol[0], pz), S_XXX, kNumSplit, lx) && lx == 0)
-                l2_prefetch(m.b + col[0] + (uint32_t)(pz + kHalo) * PL, TX * 4);
+            prefetch_split_rows(spl(), p, pml_plane_index(m, pcol[0], pz), S_XXX, kNumSplit, lx);
         }
     };
     prefetch(t.zs);
@@ -831,7 +832,8 @@ __device__ __forceinline__ bool str_item(const ZMaps &mp, const Model &m, const 
                 snew[4] = __fmaf_rn(ph.dt * mxz, xzZ + xzX, own[4 * OS + e]);
                 snew[5] = __fmaf_rn(ph.dt * myz, yzZ + yzY, own[5 * OS + e]);
             } else {
-                auto *sp = spl() + split_base32(pml_plane_index(m, pcol[c], cz));
+                const uint32_t pi = pml_plane_index(m, pcol[c], cz);
+                auto *sp = spl() + split_base32(pi);
                 constexpr uint32_t N = kSplitBlock;   // split k at sp[k * N]
                 // split S_XXX + k belongs to field txx..tyz (its scale with 16-bit storage)
                 auto grp = [](int k) { return k < 9 ? 3 + k / 3 : 6 + (k - 9) / 2; };
@@ -847,7 +849,7 @@ __device__ __forceinline__ bool str_item(const ZMaps &mp, const Model &m, const 
                 float mx = 1.f, my = 1.f, mz = 1.f;
         PDiv<FAST> px = 1, py = 1, pz = 1;
                 {
-                    const float v = damp_speed(ph, mu_c, m.b[ci], l);
+                    const float v = m.vd[pi];
                     if (kx) damp_factors<FAST>(ph, 0, ph.dx, kx, m.pml, v, mx, px);
                     if (ky) damp_factors<FAST>(ph, 1, ph.dy, ky, m.pml, v, my, py);
                     if (kz) damp_factors<FAST>(ph, 2, ph.dz, kz, m.pml, v, mz, pz);

@@ -472,11 +472,12 @@ int sgfd_create(const sgfd_config *cfg, sgfd_solver **out) {
     const size_t arr_bytes = array_bytes(m);
     const size_t pool_bytes = arr_bytes * 16;
     e = dev_malloc(h, &h->field_pool, pool_bytes);
-    if (e == cudaSuccess) e = dev_malloc(h, &h->split, (size_t)split_elems(m.npml) * sizeof(float));
+    // the splits, then the damping speeds of the PML cells
+    if (e == cudaSuccess) e = dev_malloc(h, &h->split, (size_t)(split_elems(m.npml) + m.npml) * sizeof(float));
     if (e != cudaSuccess) {
         cudaGetLastError();
         int r = fail(nullptr, SGFD_ERR_ALLOC, "device allocation of %.2f GB failed",
-                     (pool_bytes + (double)split_elems(m.npml) * 4) / 1e9);
+                     (pool_bytes + (double)(split_elems(m.npml) + m.npml) * 4) / 1e9);
         sgfd_destroy(h);
         return r;
     }
@@ -492,6 +493,7 @@ int sgfd_create(const sgfd_config *cfg, sgfd_solver **out) {
     m.b = arr(14);
     m.rmu = arr(15);
     m.split = h->split;
+    m.vd = h->split + split_elems(m.npml);
     e = cudaMemsetAsync(h->field_pool, 0, pool_bytes, h->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(h->split, 0, (size_t)split_elems(m.npml) * sizeof(float), h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
@@ -624,6 +626,7 @@ static int upload_medium(sgfd_solver *h, const float *b, const float *l, const f
     if (e == cudaSuccess)
         e = launch_shear_means(m, h->ph, const_cast<float *>(m.mxy), const_cast<float *>(m.mxz),
                                const_cast<float *>(m.myz), h->stream);
+    if (e == cudaSuccess) e = launch_damp_speed(m, h->ph, const_cast<float *>(m.vd), h->stream);
     if (e != cudaSuccess) return cuda_fail(h, e, "medium set-up kernels");
     SG_CUDA(h, cudaStreamSynchronize(h->stream), "medium upload");
     h->medium_set = true;

@@ -79,6 +79,9 @@ struct Model {
     // four mu (ElasticMacro.h:110-119), computed once per medium upload
     const float *mxy, *mxz, *myz;
     float *split;        // split_elems(npml) values, blocked (split_base)
+    // damp_speed (cell_math.cuh) of every PML cell in the compact order,
+    // computed once per medium upload
+    const float *vd;
     // z-slab of a larger model (sgfd_config.nz_total != 0): the whole model's
     // computed planes below this slab, the whole model's computed z extent,
     // and the whole model's compact index of the slab's first PML cell.  The
@@ -279,6 +282,8 @@ cudaError_t launch_reciprocal(float *rmu, const float *mu, int64_t n, cudaStream
 cudaError_t launch_pitch_rows(float *dst, int64_t px, const float *src, int nx, int64_t nrows, cudaStream_t s);
 cudaError_t launch_shear_means(const Model &m, const Physics &ph, float *mxy, float *mxz, float *myz,
                                cudaStream_t s);
+// vd[pml_index] = the damping's wave speed of every PML cell.
+cudaError_t launch_damp_speed(const Model &m, const Physics &ph, float *vd, cudaStream_t s);
 // FP64 energy audit (kernels_audit.cu): partials holds 2 doubles per block,
 // out 2 doubles (kinetic, strain).
 int energy_blocks(int num_sms);

@@ -54,7 +54,7 @@ struct sgfd_solver {
     cudaStream_t stream = nullptr;
     cudaStream_t own_stream = nullptr;
     char *field_pool = nullptr;   // 9 fields, lambda, mu, 3 shear moduli, b, 1/mu
-    float *split = nullptr;
+    float *split = nullptr;       // PML splits, then the damping speeds (Model::vd)
     int4 *rec = nullptr;
     float *traces = nullptr;
     float *wavelet = nullptr;
