@@ -298,26 +298,42 @@ int launch_step(sgfd_solver *h, int it, float value, bool use_wavelet) {
     return SGFD_OK;
 }
 
-// z chunking: chunks of at most 48 planes, shorter, down to 16 planes, when
-// the grid has too few tiles for ~16 waves of three CTAs per SM (measured on
-// B200 with 32 x 8 tiles: 24-, 32- and 48-plane chunks within 1 % on the 394^3
-// cube, 48 planes 2 % faster than 24 on the 522^3 cube, where each chunk
-// start re-reads 9 planes of the z-queued fields).
+// z chunking.  A chunk costs about 2.5 planes of start-up (filling the z
+// queues and the first stages), so long chunks waste least; short ones fill
+// the GPU when the grid has few tiles.  One wave is three CTAs on every SM
+// (measured with 32 x 8 tiles, ms per step, FP32):
+//   * every tile fits one wave with chunks of at most 14 planes: the shortest
+//     such chunk (64^3: 2 planes 0.0226, 14 planes 0.0697; 80^3: 5 planes
+//     0.0436, 14 planes 0.0711; 60 x 60 x 400: 13 planes 0.111, 8 0.122;
+//     where one wave needs longer chunks several waves are faster: 120^3
+//     16 planes 0.1261, 8 planes 0.1226);
+//   * fewer than 16 waves of 16-plane chunks: about four waves, 8 to 16
+//     planes (150^3: 8 planes 0.2161, 16 planes 0.2210; 300 x 200 x 100:
+//     12 planes 0.3443, 8 planes 0.3480, 16 planes 0.3497; 200^3 flat from 8
+//     to 16, 0.424 to 0.430);
+//   * larger grids: 16 waves, at most 48 planes (24, 32 and 48 planes within
+//     1 % on the 394^3 grid, 48 planes 2 % faster than 24 on 522^3).
 void set_zchunks(sgfd_solver *h) {
     ZGeom &g = h->zg;
-    const int tiles = g.ntx * g.nty;
+    const int tiles = g.ntx * g.nty, nz = h->m.nzc;
     int zc = h->zchunk_req;
     if (zc <= 0) {
         int sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
-        const int target = 16 * 3 * sms;
-        int nch = (target + tiles - 1) / tiles;
-        nch = std::max(1, std::min(nch, (h->m.nzc + 15) / 16));
-        zc = std::min(48, (h->m.nzc + nch - 1) / nch);
+        const int wave = 3 * sms;
+        auto chunk = [&](int waves) {
+            const int n = (waves * wave + tiles - 1) / tiles;
+            return (nz + n - 1) / n;
+        };
+        const int per_tile = wave / tiles;   // chunks of every tile that one wave holds
+        const int single = per_tile > 0 ? (nz + per_tile - 1) / per_tile : nz;
+        if (single <= 14) zc = single;
+        else if (chunk(16) < 16) zc = std::min(16, std::max(8, chunk(4)));
+        else zc = std::min(48, chunk(16));
     }
-    zc = std::max(1, std::min(zc, h->m.nzc));
+    zc = std::max(1, std::min(zc, nz));
     g.zc = zc;
-    g.nchunks = (h->m.nzc + zc - 1) / zc;
+    g.nchunks = (nz + zc - 1) / zc;
 }
 
 // Receivers bucketed per z-march tile, sorted by z (device arrays).
