@@ -108,7 +108,7 @@ typedef enum sgfd_quirks {
  * 0, 1, 3, 7, 15, 31, 49 and then every 50 steps from the largest magnitude
  * each field wrote in that step, so that it is stored near 2^7.  16-bit storage
  * runs on the z-marching kernels with 32 x 8 tiles (16-bit boxes staged by
- * TMA and widened once per plane; 64 x 8 tiles through sgfd_set_tile) or,
+ * TMA, each value widened once per update; 64 x 8 tiles through sgfd_set_tile) or,
  * with SGFD_KERNEL_SIMPLE, on the per-cell kernels; all give the same bits.
  * The per-step audit (sgfd_set_audit) is not available with it. */
 typedef enum sgfd_storage {

@@ -121,8 +121,8 @@ cudaError_t dispatch_on(sgfd_solver *h, const SourceRec &sr, cudaStream_t s, int
     cudaError_t e = h->kernel == SGFD_KERNEL_ZMARCH
                         ? (h->zg.pair ? zpair_step(h->m, h->ph, sr, h16 ? &h->hs : nullptr, h->zg, h->vm, h->sm, it,
                                                    value, use_wavelet, s, ev)
-                                      : zmarch_step(h->m, h->ph, sr, h->zg, h->zm, it, value, use_wavelet, s, ev,
-                                                    h16 ? &h->hs : nullptr))
+                           : h16 ? ztwin16_step(h->m, h->ph, sr, h->hs, h->zg, h->tm16, it, value, use_wavelet, s, ev)
+                                 : zmarch_step(h->m, h->ph, sr, h->zg, h->zm, it, value, use_wavelet, s, ev))
                     : h16 ? half_step(h->m, h->ph, sr, h->hs, it, value, use_wavelet, s, ev)
                         : simple_step(h->m, h->ph, sr, it, value, use_wavelet, s, ev);
     if (e == cudaSuccess && h->strip_n > 0)
@@ -152,6 +152,7 @@ void graph_key(const sgfd_solver *h, GraphKey *k) {
     std::memcpy(static_cast<void *>(&k->vm), &h->vm, sizeof h->vm);
     std::memcpy(static_cast<void *>(&k->sm), &h->sm, sizeof h->sm);
     std::memcpy(static_cast<void *>(&k->zm), &h->zm, sizeof h->zm);
+    std::memcpy(static_cast<void *>(&k->tm16), &h->tm16, sizeof h->tm16);
     k->kernel = h->kernel;
     k->audit_every = h->audit_every;
     k->audit_region = h->audit_region;
@@ -557,7 +558,8 @@ int sgfd_create(const sgfd_config *cfg, sgfd_solver **out) {
         h->zg.cells = 1;
         h->zg.pair = 0;
         h->zg.tw = kZTileX;
-        e = zmarch_prepare(m, h->zg.cells, arr_bytes, &h->zm, h16 ? &h->hs : nullptr, stride16(h));
+        e = h16 ? ztwin16_prepare(m, arr_bytes, h->hs, stride16(h), &h->tm16)
+                : zmarch_prepare(m, h->zg.cells, arr_bytes, &h->zm);
         if (e == cudaSuccess) e = dev_malloc(h, &h->dev_err, sizeof(int));
         if (e == cudaSuccess) e = cudaMemset(h->dev_err, 0, sizeof(int));
         if (e != cudaSuccess) {
@@ -785,8 +787,8 @@ int sgfd_step_phase_part(sgfd_solver *h, int32_t it, float source_value, int32_t
     const int phases = phase == SGFD_PHASE_VELOCITY ? 1 : 2;
     const cudaError_t e =
         h->kernel == SGFD_KERNEL_ZMARCH
-            ? zmarch_step(h->m, h->ph, h->sr, h->zg, h->zm, it, source_value, false, h->stream, nullptr, nullptr,
-                          phases, parts)
+            ? zmarch_step(h->m, h->ph, h->sr, h->zg, h->zm, it, source_value, false, h->stream, nullptr, phases,
+                          parts)
             : simple_step(h->m, h->ph, h->sr, it, source_value, false, h->stream, nullptr, phases, parts);
     if (e != cudaSuccess) return cuda_fail(h, e, "half-step launch");
     return SGFD_OK;
@@ -899,8 +901,8 @@ int sgfd_set_tile(sgfd_solver *h, int32_t tile_cols, int32_t tile_rows, int32_t 
     const int cells = tile_rows / 8;
     if (cells != h->zg.cells || (int)pair != h->zg.pair) {
         cudaError_t e = pair ? zpair_prepare(h->m, h16 ? &h->hs : nullptr, &h->vm, &h->sm)
-                             : zmarch_prepare(h->m, cells, array_bytes(h->m), &h->zm, h16 ? &h->hs : nullptr,
-                                              stride16(h));
+                        : h16 ? ztwin16_prepare(h->m, array_bytes(h->m), h->hs, stride16(h), &h->tm16)
+                              : zmarch_prepare(h->m, cells, array_bytes(h->m), &h->zm);
         if (e != cudaSuccess) return cuda_fail(h, e, "z-march re-tiling");
         h->zg.cells = cells;
         h->zg.pair = pair ? 1 : 0;

@@ -23,6 +23,7 @@ struct GraphKey {
     VelMaps vm;
     StrMaps sm;
     ZMaps zm;
+    ZTwin16Maps tm16;
     int kernel;
     int audit_every, audit_region, audit_count;
     double *audit_hist, *audit;
@@ -61,8 +62,10 @@ struct sgfd_solver {
     int wavelet_nt = 0;
     bool medium_set = false;
     int kernel = SGFD_KERNEL_SIMPLE;
-    // z-marching family: single-cell maps (zm) or paired maps (vm, sm)
+    // z-marching family: single-cell maps (FP32 storage zm, 16-bit tm16) or
+    // paired maps (vm, sm)
     sgfd::ZMaps zm{};
+    sgfd::ZTwin16Maps tm16{};
     sgfd::VelMaps vm{};
     sgfd::StrMaps sm{};
     sgfd::ZGeom zg{};

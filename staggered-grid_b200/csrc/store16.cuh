@@ -1,5 +1,5 @@
 // store16.cuh — 16-bit wavefield storage as the z-marching kernels see it
-// (kernels_zmarch.cu, kernels_zpair.cu): value h of field g reads back as
+// (kernels_ztwin16.cu, kernels_zpair.cu): value h of field g reads back as
 // float(h) * 2^e_g, and v is stored as RN16(v * 2^-e_g), binary16 saturating
 // at +-65504 — the roundings of kernels_half.cu and of the oracle.
 #pragma once

@@ -25,8 +25,15 @@ struct ZMaps {
     // z+1; own vx, vy, vz (32 x TY each)
     CUtensorMap v_sxx_sxz, v_syy_syz, v_sxy, v_b, v_lead_xz_yz, v_lead_zz, v_lead_b, v_own;
     // stress update: vx, vy, vz (48 x TY+10); lead vx + vy at z+5, vz at z+4;
-    // own txx..myz (11 arrays, 32 x TY each; with 16-bit storage the 6
-    // stored stresses in s_own and the FP32 lambda..myz in s_med)
+    // own txx..myz (11 arrays, 32 x TY each)
+    CUtensorMap s_v, s_lead_xy, s_lead_z, s_own;
+};
+
+// TMA descriptors of the 16-bit kernels that take two planes at a time
+// (kernels_ztwin16.cu): boxes two planes deep (the buoyancy three); the
+// wavefields 16-bit, the medium FP32.
+struct ZTwin16Maps {
+    CUtensorMap v_sxx_sxz, v_syy_syz, v_sxy, v_lead_xz_yz, v_lead_zz, v_own, v_b;
     CUtensorMap s_v, s_lead_xy, s_lead_z, s_own, s_med;
 };
 
@@ -66,22 +73,32 @@ struct ZGeom {
 bool make_box_map(CUtensorMap *map, const float *grid_origin, const Model &m, int bx, int by);
 bool make_box_map16(CUtensorMap *map, const uint16_t *grid_origin, const Model &m, int bx, int by);
 
+// 4-D tensor maps over `count` arrays of the pool (FP32, or the 16-bit
+// wavefields of the same layout), `stride` bytes apart, the first at `first`,
+// with a bx x by x bz x count box.
+bool make_pool_map(CUtensorMap *map, const float *first, const Model &m, size_t stride, int count, int bx, int by,
+                   int bz = 1);
+bool make_pool_map16(CUtensorMap *map, const uint16_t *first, const Model &m, size_t stride, int count, int bx, int by,
+                     int bz = 1);
+
 // zmarch_prepare: the maps of the single-cell family over the model's array
 // pool, whose arrays are array_stride bytes apart in the order the stress
-// update reads them (cudaErrorInvalidValue when the pointers are otherwise);
-// with hs (16-bit storage, cells = 1), the wavefield maps cover the 16-bit
-// arrays, stride16 bytes apart.  zmarch_step: one step (velocity + stress);
-// with hs also the 16-bit source, receiver and rescale kernels.  phases
-// (FP32 storage): bit 0 the velocity update, bit 1 the stress update; parts
-// (FP32 storage): kPartInner the z chunks whose planes read no frame plane,
-// kPartOuter the others.
+// update reads them (cudaErrorInvalidValue when the pointers are otherwise).
+// zmarch_step: one step (velocity + stress) of an FP32 handle; phases: bit 0
+// the velocity update, bit 1 the stress update; parts: kPartInner the z
+// chunks whose planes read no frame plane, kPartOuter the others.
 bool zmarch_supported(const Model &m);
-cudaError_t zmarch_prepare(const Model &m, int cells, size_t array_stride, ZMaps *zm, const HalfState *hs = nullptr,
-                           size_t stride16 = 0);
+cudaError_t zmarch_prepare(const Model &m, int cells, size_t array_stride, ZMaps *zm);
 void zmarch_tiles(const Model &m, int cells, int *ntx, int *nty);
 cudaError_t zmarch_step(const Model &m, const Physics &ph, const SourceRec &sr, const ZGeom &g, const ZMaps &zm,
                         int it, float src_value, bool use_wavelet, cudaStream_t s, cudaEvent_t *ev = nullptr,
-                        const HalfState *hs = nullptr, int phases = 3, int parts = 3);
+                        int phases = 3, int parts = 3);
+// 16-bit storage, 32 x 8 tiles (kernels_ztwin16.cu): maps and one step.
+cudaError_t ztwin16_prepare(const Model &m, size_t array_stride, const HalfState &hs, size_t stride16,
+                            ZTwin16Maps *tm);
+cudaError_t ztwin16_step(const Model &m, const Physics &ph, const SourceRec &sr, const HalfState &hs, const ZGeom &g,
+                         const ZTwin16Maps &tm, int it, float src_value, bool use_wavelet, cudaStream_t s,
+                         cudaEvent_t *ev = nullptr);
 // One model of a persistent batch, in device memory (the kernel's TMA reads
 // its tensor maps from there: 64-byte alignment).  Its work items are the
 // (tile, z chunk) pairs of the single-cell 32 x 8 tiling, tile fastest.
