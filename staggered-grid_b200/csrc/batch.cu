@@ -95,6 +95,7 @@ int capture(sgfd_batch *b) {
         sgfd_solver *h = b->models[i];
         SourceRec sr = h->sr;
         sr.it_dev = b->step_ctr;
+        sr.overlap = 0;
         for (int k = 0; k < kGraphSteps && e == cudaSuccess; ++k)
             e = dispatch_on(h, sr, b->branch[i % nb], k, 0.0f, true, nullptr);
     }

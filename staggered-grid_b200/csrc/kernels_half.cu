@@ -72,6 +72,7 @@ struct Store16 {
 // txx, tyy, tzz at the source += dt*dt*s(it), stored rounded.
 template <int ST>
 __global__ void k_inject16(Model m, Physics ph, SourceRec sr, HalfState hs, int it_arg, float value, int use_wavelet) {
+    step_wait();
     if (threadIdx.x != 0 || sr.src < 0) return;
     const int it = step_index(sr, it_arg);
     const float v = ph.inj_dt2 * (use_wavelet ? sr.wavelet[it] : value);
@@ -239,6 +240,7 @@ __global__ void __launch_bounds__(kBX * kBY) k_stress16(Model m, Physics ph, Sou
 // Receivers of one phase sample their (read-back) component.
 template <int ST>
 __global__ void k_record16(Model m, SourceRec sr, HalfState hs, int it_arg, int velocity_phase) {
+    step_wait();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     const int it = step_index(sr, it_arg);
     if (r >= sr.nrec || it < 0 || it >= sr.nt) return;
@@ -250,6 +252,7 @@ __global__ void k_record16(Model m, SourceRec sr, HalfState hs, int it_arg, int 
 // New exponents from the noted maxima (one thread); fields that noted zero
 // (or a non-finite value) keep theirs.
 __global__ void k_rescale_choose(SourceRec sr, HalfState hs, int it_arg) {
+    step_wait();
     if (threadIdx.x != 0 || !rescale_step(step_index(sr, it_arg))) return;
     for (int g = 0; g < 9; ++g) {
         const float mx = __uint_as_float(hs.amax[g]);
@@ -262,6 +265,7 @@ __global__ void k_rescale_choose(SourceRec sr, HalfState hs, int it_arg) {
 // Re-round every stored value of a field whose exponent changes.
 template <int ST>
 __global__ void k_rescale_apply(Model m, SourceRec sr, HalfState hs, int it_arg, int64_t n_grid) {
+    step_wait();
     if (!rescale_step(step_index(sr, it_arg))) return;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x, t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     // every stored value h of p[0, n) becomes RN16(float(h) * f): eight at a
@@ -312,6 +316,7 @@ __global__ void k_rescale_apply(Model m, SourceRec sr, HalfState hs, int it_arg,
 
 // Adopt the new exponents and clear the maxima for the next rescale step.
 __global__ void k_rescale_commit(SourceRec sr, HalfState hs, int it_arg) {
+    step_wait();
     if (threadIdx.x >= 9 || !rescale_step(step_index(sr, it_arg))) return;
     const int g = threadIdx.x;
     hs.e[g] = hs.e_new[g];
@@ -374,14 +379,14 @@ template <int ST>
 cudaError_t phases16(const Model &m, const Physics &ph, const SourceRec &sr, const HalfState &hs, int it,
                      float src_value, bool use_wavelet, cudaStream_t s, int phase) {
     if (phase == 0) {
-        if (sr.src >= 0) k_inject16<ST><<<1, 32, 0, s>>>(m, ph, sr, hs, it, src_value, use_wavelet ? 1 : 0);
+        if (sr.src >= 0) step_launch(k_inject16<ST>, 1, 32, 0, s, sr.overlap != 0, m, ph, sr, hs, it, src_value, use_wavelet ? 1 : 0);
     } else if (phase == 1) {
-        if (sr.nrec > 0) k_record16<ST><<<(sr.nrec + 127) / 128, 128, 0, s>>>(m, sr, hs, it, 1);
+        if (sr.nrec > 0) step_launch(k_record16<ST>, (sr.nrec + 127) / 128, 128, 0, s, sr.overlap != 0, m, sr, hs, it, 1);
     } else {
-        if (sr.nrec > 0) k_record16<ST><<<(sr.nrec + 127) / 128, 128, 0, s>>>(m, sr, hs, it, 0);
-        k_rescale_choose<<<1, 32, 0, s>>>(sr, hs, it);
-        k_rescale_apply<ST><<<1184, 256, 0, s>>>(m, sr, hs, it, m.plane * m.nz);
-        k_rescale_commit<<<1, 32, 0, s>>>(sr, hs, it);
+        if (sr.nrec > 0) step_launch(k_record16<ST>, (sr.nrec + 127) / 128, 128, 0, s, sr.overlap != 0, m, sr, hs, it, 0);
+        step_launch(k_rescale_choose, 1, 32, 0, s, sr.overlap != 0, sr, hs, it);
+        step_launch(k_rescale_apply<ST>, 1184, 256, 0, s, sr.overlap != 0, m, sr, hs, it, m.plane * m.nz);
+        step_launch(k_rescale_commit, 1, 32, 0, s, sr.overlap != 0, sr, hs, it);
     }
     return cudaGetLastError();
 }

@@ -472,6 +472,7 @@ k_velocity_zmarch(const __grid_constant__ ZMaps mp, const __grid_constant__ Mode
         fence_barrier_init();
     }
     __syncthreads();
+    step_wait();
     uint32_t pbits = 0;
     vel_item<FAST, CELLS, false>(mp, m, ph, g, sr, it_arg, src_value, use_wavelet, blockIdx.x, blockIdx.y + g.c0,
                           align_smem(smem_raw), bar, boxes, pbits);
@@ -785,6 +786,7 @@ k_stress_zmarch(const __grid_constant__ ZMaps mp, const __grid_constant__ Model 
         fence_barrier_init();
     }
     __syncthreads();
+    step_wait();
     uint32_t pbits = 0;
     str_item<FAST, CELLS, false>(mp, m, ph, g, sr, it_arg, src_value, use_wavelet, blockIdx.x, blockIdx.y + g.c0,
                           align_smem(smem_raw), bar, boxes, pbits);
@@ -925,14 +927,16 @@ void launch(const Model &m, const Physics &ph, const SourceRec &sr, const ZGeom 
     if (phases & 1) {
         if (ev) cudaEventRecord(ev[0], s);
         each([&](dim3 grid, const ZGeom &gr) {
-            k_velocity_zmarch<FAST, CELLS><<<grid, NT, vel_smem<CELLS>(), s>>>(zm, m, ph, gr, sr, it, src_value, uw);
+            step_launch(k_velocity_zmarch<FAST, CELLS>, grid, NT, vel_smem<CELLS>(), s, sr.overlap != 0, zm, m, ph, gr,
+                        sr, it, src_value, uw);
         });
         if (ev) cudaEventRecord(ev[1], s);
     }
     if (phases & 2) {
         if (ev) cudaEventRecord(ev[2], s);
         each([&](dim3 grid, const ZGeom &gr) {
-            k_stress_zmarch<FAST, CELLS><<<grid, NT, str_smem<CELLS>(), s>>>(zm, m, ph, gr, sr, it, src_value, uw);
+            step_launch(k_stress_zmarch<FAST, CELLS>, grid, NT, str_smem<CELLS>(), s, sr.overlap != 0, zm, m, ph, gr,
+                        sr, it, src_value, uw);
         });
         if (ev) cudaEventRecord(ev[3], s);
     }

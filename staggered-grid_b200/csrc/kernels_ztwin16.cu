@@ -115,6 +115,7 @@ __device__ __forceinline__ void init16(Shared16 &y, const HalfState &hs) {
         mbar_init(&y.own, 1);
         fence_barrier_init();
     }
+    step_wait();
     if (threadIdx.x < 9) {
         y.scl[threadIdx.x] = hs.sc[threadIdx.x];
         y.scl[9 + threadIdx.x] = hs.inv[threadIdx.x];
@@ -670,11 +671,11 @@ void launch(const Model &m, const Physics &ph, const SourceRec &sr, const HalfSt
     const dim3 grid(g.ntx * g.nty, g.nchunks);
     half_phase(m, ph, sr, hs, it, src_value, uw, s, 0);
     if (ev) cudaEventRecord(ev[0], s);
-    k_velocity_ztwin16<FAST, ST><<<grid, NT, smem_bytes<VelH>(), s>>>(tm, m, ph, g, sr, hs, it);
+    step_launch(k_velocity_ztwin16<FAST, ST>, grid, NT, smem_bytes<VelH>(), s, sr.overlap != 0, tm, m, ph, g, sr, hs, it);
     if (ev) cudaEventRecord(ev[1], s);
     half_phase(m, ph, sr, hs, it, src_value, uw, s, 1);
     if (ev) cudaEventRecord(ev[2], s);
-    k_stress_ztwin16<FAST, ST><<<grid, NT, smem_bytes<StrH>(), s>>>(tm, m, ph, g, sr, hs, it);
+    step_launch(k_stress_ztwin16<FAST, ST>, grid, NT, smem_bytes<StrH>(), s, sr.overlap != 0, tm, m, ph, g, sr, hs, it);
     if (ev) cudaEventRecord(ev[3], s);
     half_phase(m, ph, sr, hs, it, src_value, uw, s, 2);
 }

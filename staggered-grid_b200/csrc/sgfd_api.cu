@@ -267,6 +267,7 @@ int capture_graph(sgfd_solver *h) {
     }
     SourceRec sr = h->sr;
     sr.it_dev = h->step_ctr;
+    if (h->storage == SGFD_STORE_F32) sr.overlap = 0;   // replays have no launch latency to hide
     SG_CUDA(h, cudaStreamBeginCapture(h->cap_stream, cudaStreamCaptureModeThreadLocal), "begin capture");
     cudaError_t e = cudaSuccess;
     for (int k = 0; k < kGraphSteps && e == cudaSuccess; ++k)
@@ -319,9 +320,7 @@ void set_zchunks(sgfd_solver *h) {
     const int tiles = g.ntx * g.nty, nz = h->m.nzc;
     int zc = h->zchunk_req;
     if (zc <= 0) {
-        int sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
-        const int wave = 3 * sms;
+        const int wave = 3 * h->sms;
         auto chunk = [&](int waves) {
             const int n = (waves * wave + tiles - 1) / tiles;
             return (nz + n - 1) / n;
@@ -335,6 +334,9 @@ void set_zchunks(sgfd_solver *h) {
     zc = std::max(1, std::min(zc, nz));
     g.zc = zc;
     g.nchunks = (nz + zc - 1) / zc;
+    // launches overlap (step_launch) where their latency shows: the eight
+    // launches of a 16-bit step, and grids of at most one wave
+    h->sr.overlap = h->storage != SGFD_STORE_F32 || (int64_t)tiles * g.nchunks <= 3 * h->sms;
 }
 
 // Receivers bucketed per z-march tile, sorted by z (device arrays).
@@ -469,6 +471,7 @@ int sgfd_create(const sgfd_config *cfg, sgfd_solver **out) {
     h->kernel = SGFD_KERNEL_SIMPLE;
     cudaError_t e = cudaSetDevice(h->device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device);
     if (e != cudaSuccess) {
         int r = cuda_fail(nullptr, e, "device setup");
         delete h;
@@ -785,11 +788,13 @@ int sgfd_step_phase_part(sgfd_solver *h, int32_t it, float source_value, int32_t
     if (h->strip_n > 0 || h->audit_every > 0)
         return fail(h, SGFD_ERR_UNSUPPORTED, "half steps run neither a learned strip nor a per-step audit");
     const int phases = phase == SGFD_PHASE_VELOCITY ? 1 : 2;
+    SourceRec sr = h->sr;
+    sr.overlap = 0;   // the slabs of a model share the GPU
     const cudaError_t e =
         h->kernel == SGFD_KERNEL_ZMARCH
-            ? zmarch_step(h->m, h->ph, h->sr, h->zg, h->zm, it, source_value, false, h->stream, nullptr, phases,
+            ? zmarch_step(h->m, h->ph, sr, h->zg, h->zm, it, source_value, false, h->stream, nullptr, phases,
                           parts)
-            : simple_step(h->m, h->ph, h->sr, it, source_value, false, h->stream, nullptr, phases, parts);
+            : simple_step(h->m, h->ph, sr, it, source_value, false, h->stream, nullptr, phases, parts);
     if (e != cudaSuccess) return cuda_fail(h, e, "half-step launch");
     return SGFD_OK;
 }

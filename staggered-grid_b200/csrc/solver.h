@@ -52,6 +52,7 @@ struct sgfd_solver {
     sgfd::Physics ph{};
     sgfd::SourceRec sr{};
     int device = 0;
+    int sms = 148;                // the device's SM count
     cudaStream_t stream = nullptr;
     cudaStream_t own_stream = nullptr;
     char *field_pool = nullptr;   // 9 fields, lambda, mu, 3 shear moduli, b, 1/mu
