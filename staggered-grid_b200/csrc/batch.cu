@@ -38,6 +38,7 @@ struct sgfd_batch {
     // persistent mode: one cooperative launch runs every model's work items
     bool persistent = false;
     bool pfast = false;
+    bool psame = false;                   // every model has the first one's physics
     int barrier_ctas = 0;                 // 0: as many as launched
     int ctas = 0;                         // CTAs that fit at once
     ZModel *pdesc = nullptr;              // device copies of the models' descriptors
@@ -140,12 +141,14 @@ int build_descriptors(sgfd_batch *b) {
     if (current) return SGFD_OK;
     std::vector<ZModel> d(n);
     std::vector<int> first(n + 1, 0);
+    b->psame = true;
     for (int i = 0; i < n; ++i) {
         const sgfd_solver *h = b->models[i];
         std::memset(static_cast<void *>(&d[i]), 0, sizeof d[i]);
         d[i].zm = h->zm;
         d[i].m = h->m;
         d[i].ph = h->ph;
+        b->psame = b->psame && std::memcmp(&h->ph, &b->models[0]->ph, sizeof h->ph) == 0;
         d[i].g = h->zg;
         d[i].sr = h->sr;
         d[i].sr.it_dev = nullptr;
@@ -189,7 +192,7 @@ int run_persistent(sgfd_batch *b, int it0, int nsteps) {
                "batch counters");
     const int bar = b->barrier_ctas > 0 ? b->barrier_ctas : b->ctas;
     BATCH_CUDA(b, zmarch_batch_run(b->pdesc, (int)b->models.size(), b->pfirst, it0, nsteps, b->pctl, bar, b->ctas,
-                                   b->pfast, b->pstatus, b->stream),
+                                   b->models[0]->ph, b->psame, b->pstatus, b->stream),
                "persistent batch launch");
     return SGFD_OK;
 }

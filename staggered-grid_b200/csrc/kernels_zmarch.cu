@@ -49,6 +49,7 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include <climits>
 #include <type_traits>
 
 #include "cell_math.cuh"
@@ -827,8 +828,9 @@ cudaError_t set_attrs() {
 
 constexpr int batch_smem() { return vel_smem<1>() > str_smem<1>() ? vel_smem<1>() : str_smem<1>(); }
 
-// The two updates as called functions, so that each is register-allocated on
-// its own rather than inlined side by side into the persistent loop.
+// The two updates as called functions, for models of differing physics: each
+// is register-allocated on its own rather than inlined side by side into the
+// persistent loop.
 template <bool FAST>
 __device__ __noinline__ bool vel_item_call(const ZMaps &mp, const Model &m, const Physics &ph, const ZGeom &g,
                                            const SourceRec &sr, int it, int tile, int chunk, unsigned char *smem,
@@ -842,21 +844,26 @@ __device__ __noinline__ bool str_item_call(const ZMaps &mp, const Model &m, cons
     return str_item<FAST, 1, true>(mp, m, ph, g, sr, it, 0.0f, 1, tile, chunk, smem, bar, boxes, pbits);
 }
 
-// Two CTAs per SM: the 128 registers a thread then has keep both called
-// updates nearly free of spills (at three CTAs the stress update, whose
-// physics and geometry come from shared memory here, spills 0.5 KB).
-template <bool FAST>
+// SAME: all models have the same physics (ph), as the models of one survey
+// do; the updates, inlined, then take their constants from the constant bank
+// as single launches do.  Otherwise each model's physics is copied to shared
+// memory, read there in every plane's inner loops (12 models of 146^3 to
+// 306^3, 16 steps: 135.5 ms that way, 126.7 ms with SAME).
+// Two CTAs per SM: with the 80 registers a thread of three CTAs both updates
+// spill beside the loop's own state (SAME 145.8 ms, called 171.4 ms).
+template <bool FAST, bool SAME>
 __global__ void __launch_bounds__(NT, 2)
 k_batch_zmarch(const ZModel *models, int nmodels, const int *first_item, int it0, int nsteps, unsigned *ctl,
-               unsigned barrier_ctas, int *status) {
+               unsigned barrier_ctas, int *status, const __grid_constant__ Physics ph) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar_v[S];
     __shared__ __align__(8) uint64_t bar_s[S];
     __shared__ TmaBox boxes[kWarps][kMaxBoxesPerWarp];
     __shared__ int item_sh, ok_sh;
-    // the current model's physics and geometry, read in every plane's inner
-    // loops: a shared copy instead of loads from the descriptor array
-    __shared__ __align__(16) Physics ph_s;
+    // the current model's geometry (and physics): a shared copy instead of
+    // loads from the descriptor array
+    __shared__ __align__(16) unsigned char ph_raw[SAME ? 16 : sizeof(Physics)];
+    [[maybe_unused]] Physics &ph_s = *reinterpret_cast<Physics *>(ph_raw);
     __shared__ __align__(16) Model m_s;
     int cur = -1;
     if (threadIdx.x == 0) {
@@ -882,22 +889,29 @@ k_batch_zmarch(const ZModel *models, int nmodels, const int *first_item, int it0
                 while (first_item[mi + 1] <= item) ++mi;
                 const ZModel &d = models[mi];
                 if (mi != cur) {   // every thread is past the previous item (the barriers above)
-                    const uint32_t *src = reinterpret_cast<const uint32_t *>(&d.ph);
-                    uint32_t *dst = reinterpret_cast<uint32_t *>(&ph_s);
-                    for (int i = threadIdx.x; i < (int)(sizeof(Physics) / 4); i += NT) dst[i] = src[i];
-                    src = reinterpret_cast<const uint32_t *>(&d.m);
-                    dst = reinterpret_cast<uint32_t *>(&m_s);
-                    for (int i = threadIdx.x; i < (int)(sizeof(Model) / 4); i += NT) dst[i] = src[i];
+                    auto copy = [](void *dst, const void *src, int words) {
+                        for (int i = threadIdx.x; i < words; i += NT)
+                            static_cast<uint32_t *>(dst)[i] = static_cast<const uint32_t *>(src)[i];
+                    };
+                    if constexpr (!SAME) copy(&ph_s, &d.ph, sizeof(Physics) / 4);
+                    copy(&m_s, &d.m, sizeof(Model) / 4);
                     __syncthreads();
                     cur = mi;
                 }
                 const int local = item - first_item[mi];
                 const int ntiles = d.g.ntx * d.g.nty;
-                const bool ok =
-                    p == 0 ? vel_item_call<FAST>(d.zm, m_s, ph_s, d.g, d.sr, it0 + k, local % ntiles, local / ntiles,
-                                                 smem, bar_v, boxes, pv)
-                           : str_item_call<FAST>(d.zm, m_s, ph_s, d.g, d.sr, it0 + k, local % ntiles, local / ntiles,
-                                                 smem, bar_s, boxes, ps);
+                const int tile = local % ntiles, chunk = local / ntiles;
+                bool ok;
+                if constexpr (SAME)
+                    ok = p == 0 ? vel_item<FAST, 1, true>(d.zm, m_s, ph, d.g, d.sr, it0 + k, 0.0f, 1, tile, chunk, smem,
+                                                          bar_v, boxes, pv)
+                                : str_item<FAST, 1, true>(d.zm, m_s, ph, d.g, d.sr, it0 + k, 0.0f, 1, tile, chunk, smem,
+                                                          bar_s, boxes, ps);
+                else
+                    ok = p == 0 ? vel_item_call<FAST>(d.zm, m_s, ph_s, d.g, d.sr, it0 + k, tile, chunk, smem, bar_v,
+                                                      boxes, pv)
+                                : str_item_call<FAST>(d.zm, m_s, ph_s, d.g, d.sr, it0 + k, tile, chunk, smem, bar_s,
+                                                      boxes, ps);
                 if (!ok) {
                     if (threadIdx.x == 0) atomicExch(status, kBatchWaitTma);
                     return;
@@ -1059,27 +1073,32 @@ cudaError_t zmarch_step(const Model &m, const Physics &ph, const SourceRec &sr, 
     return cudaGetLastError();
 }
 
+static const void *batch_kernel(bool fast, bool same) {
+    return fast ? (same ? (const void *)k_batch_zmarch<true, true> : (const void *)k_batch_zmarch<true, false>)
+                : (same ? (const void *)k_batch_zmarch<false, true> : (const void *)k_batch_zmarch<false, false>);
+}
+
 int zmarch_batch_ctas(int device) {
-    int sms = 0, per = 0, per2 = 0;
+    int sms = 0, fit = INT_MAX;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
-    if (cudaFuncSetAttribute(k_batch_zmarch<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, batch_smem()) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(k_batch_zmarch<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, batch_smem()) !=
-            cudaSuccess)
-        return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch_zmarch<true>, NT, batch_smem()) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, k_batch_zmarch<false>, NT, batch_smem()) != cudaSuccess)
-        return 0;
-    return sms * (per < per2 ? per : per2);
+    for (int v = 0; v < 4; ++v) {
+        const void *fn = batch_kernel(v & 1, v & 2);
+        int per = 0;
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, batch_smem()) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, NT, batch_smem()) != cudaSuccess)
+            return 0;
+        fit = per < fit ? per : fit;
+    }
+    return sms * fit;
 }
 
 cudaError_t zmarch_batch_run(const ZModel *models, int nmodels, const int *first_item, int it0, int nsteps,
-                             unsigned *ctl, int barrier_ctas, int ctas, bool fast, int *status, cudaStream_t s) {
+                             unsigned *ctl, int barrier_ctas, int ctas, const Physics &ph, bool same, int *status,
+                             cudaStream_t s) {
     unsigned target = (unsigned)barrier_ctas;
-    void *args[] = {(void *)&models, (void *)&nmodels, (void *)&first_item, (void *)&it0, (void *)&nsteps,
-                    (void *)&ctl, (void *)&target, (void *)&status};
-    const void *fn = fast ? (const void *)k_batch_zmarch<true> : (const void *)k_batch_zmarch<false>;
-    return cudaLaunchCooperativeKernel(fn, dim3(ctas), dim3(NT), args, batch_smem(), s);
+    void *args[] = {(void *)&models, (void *)&nmodels, (void *)&first_item, (void *)&it0,   (void *)&nsteps,
+                    (void *)&ctl,    (void *)&target,  (void *)&status,     (void *)&ph};
+    return cudaLaunchCooperativeKernel(batch_kernel(ph.fast, same), dim3(ctas), dim3(NT), args, batch_smem(), s);
 }
 
 }  // namespace sgfd

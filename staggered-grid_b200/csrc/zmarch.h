@@ -120,10 +120,12 @@ constexpr int kBatchWaitTma = 1, kBatchWaitGrid = 2;
 // (grid-barrier arrivals, then one work counter per step and phase); each
 // grid barrier waits for barrier_ctas arrivals (the launched CTAs unless a
 // caller asks otherwise), at most about a second, then the launch stops with
-// *status = kBatchWaitGrid.  All models FAST or all REF (fast).
+// *status = kBatchWaitGrid.  All models FAST or all REF; ph: the first
+// model's physics; same: every model's physics equals it.
 int zmarch_batch_ctas(int device);
 cudaError_t zmarch_batch_run(const ZModel *models, int nmodels, const int *first_item, int it0, int nsteps,
-                             unsigned *ctl, int barrier_ctas, int ctas, bool fast, int *status, cudaStream_t s);
+                             unsigned *ctl, int barrier_ctas, int ctas, const Physics &ph, bool same, int *status,
+                             cudaStream_t s);
 
 // Paired tiling: tensor maps, tile counts and one step (velocity + stress).
 // hs: null for FP32 storage, else the 16-bit storage state (the step then
