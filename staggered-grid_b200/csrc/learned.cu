@@ -414,15 +414,24 @@ __device__ __forceinline__ void staged_inputs(const float *stg, int c0, int sx, 
     for (int j = J0; j < J0 + 8; ++j) {
         float v[8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int f = 8 * j + q;
-            if (f < 243) {
-                const int n = f / 9, k = f % 9;
-                const int o = c0 + (n % 3 - 1) + ((n / 3) % 3 - 1) * sx + (n / 9 - 1) * sxy;
-                v[q] = stg[k * kStage + o] * (k < 3 ? zinv : inv);
-            } else {
-                v[q] = f < kIn ? ext[f - 243] : 0.0f;
+        for (int q = 0; q < 8; q += 2) {   // two inputs per packed multiplication
+            float a[2], b[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int f = 8 * j + q + e;
+                if (f < 243) {
+                    const int n = f / 9, k = f % 9;
+                    const int o = c0 + (n % 3 - 1) + ((n / 3) % 3 - 1) * sx + (n / 9 - 1) * sxy;
+                    a[e] = stg[k * kStage + o];
+                    b[e] = k < 3 ? zinv : inv;
+                } else {
+                    a[e] = f < kIn ? ext[f - 243] : 0.0f;
+                    b[e] = 1.0f;
+                }
             }
+            const float2 r = __fmul2_rn(make_float2(a[0], a[1]), make_float2(b[0], b[1]));
+            v[q] = r.x;
+            v[q + 1] = r.y;
         }
         store_chunk(a_op + kmaj(t, col0 + 8 * (j - J0), kKHalf), v);
     }
@@ -471,7 +480,9 @@ k_strip_tc(Model m, int w, const int4 *tiles, int ntiles, const unsigned char *w
     const float *b1 = reinterpret_cast<const float *>(sm + kImgB), *b2 = b1 + kH, *b3 = b2 + kH;
     uint64_t *mybar = &bar[g];
     uint32_t parity = 0;
-    bool failed = false;
+    // bad: this thread's wait for its tensor-core results gave up; the group
+    // votes on it at its next barrier, before anything else is issued
+    bool failed = false, bad = false;
 
     const int nt = ROWS ? (int)((nrows + kRows - 1) / kRows) : ntiles;
     const int first = kGroups * (int)blockIdx.x + g, stride = kGroups * (int)gridDim.x;
@@ -497,7 +508,7 @@ k_strip_tc(Model m, int w, const int4 *tiles, int ntiles, const unsigned char *w
                 stg[9 * kStage + r] = sq_velocity(f);
                 stg[10 * kStage + r] = sq_stress(f);
             }
-            wg_sync(g);
+            if (wg_sync_or(g, bad)) { failed = true; break; }
             count = bx.ex * bx.ey * bx.ez;
             if (t < count) {
                 const int lx = t % bx.ex, ly = (t / bx.ex) % bx.ey, lz = t / (bx.ex * bx.ey);
@@ -531,7 +542,6 @@ k_strip_tc(Model m, int w, const int4 *tiles, int ntiles, const unsigned char *w
 
         // ---- layer 1 in two halves of K: D1 = A W1^T, the A operand holding
         // inputs 128*half .. 128*half+127 (row t: 64 of them per thread) ----
-        bool bad = false;
         for (int half = 0; half < 2; ++half) {
             if (ROWS) {
                 const float *x = X + ((int64_t)tile * kRows + t) * kIn;
@@ -568,7 +578,7 @@ k_strip_tc(Model m, int w, const int4 *tiles, int ntiles, const unsigned char *w
             }
             fence_async_smem();
             tc_before();
-            wg_sync(g);
+            if (wg_sync_or(g, bad)) { failed = true; break; }
             if (u == 0) {
                 tc_after();
                 mma_k(tmem_g, a_s, kKHalf, w1_s + half * (kKHalf / 16) * 256, kK1, kKHalf / 16, kH, half > 0);
@@ -577,42 +587,40 @@ k_strip_tc(Model m, int w, const int4 *tiles, int ntiles, const unsigned char *w
             // after the second half the staging area is free: the next tile's
             // copies overlap this one's network
             if (!ROWS && half == 1 && tile + stride < nt) stage_async(m, tiles[tile + stride], stg, med, u);
-            const bool ok = mbar_wait_bounded(mybar, parity);
+            // no barrier here: a thread that has seen the commit may overwrite
+            // the A operand and read its own accumulators
+            bad = !mbar_wait_bounded(mybar, parity);
             parity ^= 1u;
-            bad = wg_sync_or(g, !ok);
-            if (bad) break;
             tc_after();
         }
-        if (bad) { failed = true; break; }
+        if (failed) break;
         hidden_half(tmem, b1, a_op, t, 32 * h);
 
         // ---- layer 2: D2 = H1 (128 x 64) W2^T ----
         fence_async_smem();
         tc_before();
-        wg_sync(g);
+        if (wg_sync_or(g, bad)) { failed = true; break; }
         if (u == 0) {
             tc_after();
             mma_chain(tmem_g + 64, a_s, w2_s, kH, kH);
             mma_commit(mybar);
         }
-        bool ok = mbar_wait_bounded(mybar, parity);
+        bad = !mbar_wait_bounded(mybar, parity);
         parity ^= 1u;
-        if (wg_sync_or(g, !ok)) { failed = true; break; }
         tc_after();
         hidden_half(tmem + 64, b2, a_op, t, 32 * h);
 
         // ---- layer 3: D3 = H2 (128 x 64) W3^T, N = 16 ----
         fence_async_smem();
         tc_before();
-        wg_sync(g);
+        if (wg_sync_or(g, bad)) { failed = true; break; }
         if (u == 0) {
             tc_after();
             mma_chain(tmem_g, a_s, w3_s, kH, kN3);
             mma_commit(mybar);
         }
-        ok = mbar_wait_bounded(mybar, parity);
+        bad = !mbar_wait_bounded(mybar, parity);
         parity ^= 1u;
-        if (wg_sync_or(g, !ok)) { failed = true; break; }
         tc_after();
 
         // ---- epilogue (half 0) ----
@@ -652,6 +660,7 @@ k_strip_tc(Model m, int w, const int4 *tiles, int ntiles, const unsigned char *w
         }
     }
     cp_async_wait_all();
+    if (!failed) failed = wg_sync_or(g, bad);   // the last tile's vote
     if (failed) {
         if (u == 0) atomicOr(err, 4);
         mbar_wait_bounded(mybar, parity ^ 1u);   // the commit the failed wait was for
@@ -674,14 +683,16 @@ int tc_grid(int ntiles) {
 
 // Writes the corrected fields into the strip cells (after every cell's
 // correction has been computed from the uncorrected state).  One block per
-// tile; k_strip_tc left f + a d for each cell in delta[tile][k][128].
+// tile; k_strip_tc left f + a d for each cell in delta[tile][k][128].  Last
+// tiles first: their corrections, written last, are still in L2.
 __global__ void __launch_bounds__(kRows) k_strip_apply(Model m, const int4 *tiles, const float *delta) {
-    const Box bx = box_of(tiles[blockIdx.x]);
+    const int tile = (int)(gridDim.x - 1 - blockIdx.x);
+    const Box bx = box_of(tiles[tile]);
     const int t = threadIdx.x;
     if (t >= bx.ex * bx.ey * bx.ez) return;
     const int lx = t % bx.ex, ly = (t / bx.ex) % bx.ey, lz = t / (bx.ex * bx.ey);
     const int64_t c = pidx(m, bx.x + lx + kHalo, bx.y + ly + kHalo, bx.z + lz + kHalo);
-    const float *dt = delta + (int64_t)blockIdx.x * (kRows * kOut);
+    const float *dt = delta + (int64_t)tile * (kRows * kOut);
     float v[kOut];   // every load before the first store (the arrays could alias as far as the compiler knows)
 #pragma unroll
     for (int k = 0; k < kOut; ++k) v[k] = dt[k * kRows + t];
