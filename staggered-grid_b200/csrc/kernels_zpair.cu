@@ -497,9 +497,9 @@ __device__ __forceinline__ bool vel_pair(const VelMaps &mp, const Model &m, cons
                 SA::put2(F.f(1) + ci, v1, bcast(F.inv(1)), pc.act1);
                 SA::put2(F.f(2) + ci, v2, bcast(F.inv(2)), pc.act1);
                 if (track) {
-                    note_max16s(smax, 0, fmaxf(fabsf(v0.x), pc.act1 ? fabsf(v0.y) : 0.0f));
-                    note_max16s(smax, 1, fmaxf(fabsf(v1.x), pc.act1 ? fabsf(v1.y) : 0.0f));
-                    note_max16s(smax, 2, fmaxf(fabsf(v2.x), pc.act1 ? fabsf(v2.y) : 0.0f));
+                    note_max16s(smax, 0, v0, pc.act1);
+                    note_max16s(smax, 1, v1, pc.act1);
+                    note_max16s(smax, 2, v2, pc.act1);
                 }
             } else {
                 // general path, cell by cell; PML cells through their split fields
@@ -754,7 +754,7 @@ __device__ __forceinline__ bool str_pair(const StrMaps &mp, const Model &m, cons
 #pragma unroll
                 for (int q = 0; q < 6; ++q) {
                     SA::put2(F.f(3 + q) + ci, sn[q], bcast(F.inv(3 + q)), pc.act1);
-                    if (track) note_max16s(smax, 3 + q, fmaxf(fabsf(sn[q].x), pc.act1 ? fabsf(sn[q].y) : 0.0f));
+                    if (track) note_max16s(smax, 3 + q, sn[q], pc.act1);
                 }
             } else {
 #pragma unroll

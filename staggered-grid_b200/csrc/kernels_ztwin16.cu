@@ -537,7 +537,7 @@ k_stress_ztwin16(const __grid_constant__ ZTwin16Maps mp, const __grid_constant__
             auto store = [&](int q, float2 v) {
                 if (!c.act) return;
                 uint16_t *p = hs.f[3 + q] + ci;
-                if (track) note_max16s(y.smax, 3 + q, fmaxf(fabsf(v.x), second ? fabsf(v.y) : 0.0f));
+                if (track) note_max16s(y.smax, 3 + q, v, second);
                 put(p, 3 + q, v.x);
                 if (second) put(p + PL, 3 + q, v.y);
             };

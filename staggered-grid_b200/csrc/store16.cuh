@@ -36,10 +36,19 @@ __device__ __forceinline__ void note_max16(const HalfState &hs, int g, float v) 
 
 // The same into a CTA's shared running maxima (smax[g], unsigned float
 // bits); the CTA adds them to the global ones once (flush_max16).
-__device__ __forceinline__ void note_max16s(unsigned *smax, int g, float v) {
+__device__ __forceinline__ void note_bits16s(unsigned *smax, int g, unsigned v) {
     const unsigned mask = __activemask();
-    const unsigned bits = __reduce_max_sync(mask, __float_as_uint(fabsf(v)));
+    const unsigned bits = __reduce_max_sync(mask, v);
     if ((threadIdx.x & 31) == __ffs(mask) - 1) atomicMax(smax + g, bits);
+}
+__device__ __forceinline__ void note_max16s(unsigned *smax, int g, float v) {
+    note_bits16s(smax, g, __float_as_uint(fabsf(v)));
+}
+// Two values at once (the second only if `second`), compared as bits: fmaxf
+// would drop a NaN, whose bits are the largest and keep the field's exponent.
+__device__ __forceinline__ void note_max16s(unsigned *smax, int g, float2 v, bool second) {
+    const unsigned a = __float_as_uint(fabsf(v.x)), b = second ? __float_as_uint(fabsf(v.y)) : 0u;
+    note_bits16s(smax, g, a > b ? a : b);
 }
 // After a barrier: threads 0..8 add the CTA's maxima to the global ones.
 __device__ __forceinline__ void flush_max16(const HalfState &hs, const unsigned *smax) {
