@@ -218,16 +218,31 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// Bounded wait for a group's commit, after which its accumulators may be read
+// (false: gave up); flips parity.  Every lane polls by itself, and lane 0 of
+// the group's first warp has issued the MMAs by itself: the warp meets again
+// here, because the TMEM loads that follow are warp-wide (.sync.aligned).
+__device__ __forceinline__ bool wait_commit(uint64_t *bar, uint32_t &parity) {
+    const bool ok = mbar_wait_bounded(bar, parity);
+    parity ^= 1u;
+    __syncwarp();
+    tc_after();
+    return ok;
+}
 // Barrier of one 256-thread warpgroup pair (named barrier 1 + g) that also
-// ORs a flag over it.
+// ORs a flag over it.  (bar.sync and bar.red are warp-wide too.)
 __device__ __forceinline__ bool wg_sync_or(int g, bool flag) {
     uint32_t r;
+    __syncwarp();
     asm volatile(
         "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.or.pred q, %2, 256, p;\n selp.u32 %0, 1, 0, q;\n}\n"
         : "=r"(r) : "r"((uint32_t)flag), "r"(g + 1) : "memory");
     return r != 0;
 }
-__device__ __forceinline__ void wg_sync(int g) { asm volatile("bar.sync %0, 256;" ::"r"(g + 1) : "memory"); }
+__device__ __forceinline__ void wg_sync(int g) {
+    __syncwarp();
+    asm volatile("bar.sync %0, 256;" ::"r"(g + 1) : "memory");
+}
 
 // D[tmem] (+)= A[a] * B[b]^T over nk steps of K = 16 (M = 128, N = n); A and
 // B are K-major with kta and ktb columns; acc: add to D from the first step.
@@ -470,6 +485,7 @@ k_strip_tc(Model m, int w, const int4 *tiles, int ntiles, const unsigned char *w
         reinterpret_cast<uint4 *>(sm)[i] = reinterpret_cast<const uint4 *>(wimg)[i];
     if (tid < kGroups) mbar_init1(&bar[tid]);
     if (warp == 0) {
+        __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr_of(tmem_slot)),
                      "r"(kTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -595,9 +611,7 @@ k_strip_tc(Model m, int w, const int4 *tiles, int ntiles, const unsigned char *w
             if (!ROWS && half == 1 && tile + stride < nt) stage_async(m, tiles[tile + stride], stg, med, u);
             // no barrier here: a thread that has seen the commit may overwrite
             // the A operand and read its own accumulators
-            bad = !mbar_wait_bounded(mybar, parity);
-            parity ^= 1u;
-            tc_after();
+            bad = !wait_commit(mybar, parity);
         }
         if (failed) break;
         hidden_half(tmem, b1, a_op, t, 32 * h);
@@ -611,9 +625,7 @@ k_strip_tc(Model m, int w, const int4 *tiles, int ntiles, const unsigned char *w
             mma_chain(tmem_g + 64, a_s, w2_s, kH, kH);
             mma_commit(mybar);
         }
-        bad = !mbar_wait_bounded(mybar, parity);
-        parity ^= 1u;
-        tc_after();
+        bad = !wait_commit(mybar, parity);
         hidden_half(tmem + 64, b2, a_op, t, 32 * h);
 
         // ---- layer 3: D3 = H2 (128 x 64) W3^T, N = 16 ----
@@ -625,9 +637,7 @@ k_strip_tc(Model m, int w, const int4 *tiles, int ntiles, const unsigned char *w
             mma_chain(tmem_g, a_s, w3_s, kH, kN3);
             mma_commit(mybar);
         }
-        bad = !mbar_wait_bounded(mybar, parity);
-        parity ^= 1u;
-        tc_after();
+        bad = !wait_commit(mybar, parity);
 
         // ---- epilogue (half 0) ----
         if (h == 0) {
@@ -674,6 +684,7 @@ k_strip_tc(Model m, int w, const int4 *tiles, int ntiles, const unsigned char *w
     tc_before();
     __syncthreads();
     if (warp == 0) {
+        __syncwarp();
         tc_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols)
                      : "memory");
