@@ -86,19 +86,29 @@ bool keys_current(const sgfd_batch *b) {
     return true;
 }
 
+// Tiles of all z-marching models.
+int64_t batch_tiles(const sgfd_batch *b, bool persistent) {
+    int64_t n = 0;
+    for (const sgfd_solver *h : b->models)
+        if (persistent || h->kernel == SGFD_KERNEL_ZMARCH) n += (int64_t)h->zg.ntx * h->zg.nty;
+    return std::max<int64_t>(n, 1);
+}
+
 int capture(sgfd_batch *b) {
     release(b);
     BATCH_CUDA(b, cudaStreamBeginCapture(b->cap, cudaStreamCaptureModeThreadLocal), "begin capture");
     cudaError_t e = cudaEventRecord(b->fork, b->cap);
     const int nb = (int)b->branch.size();
+    const int64_t tiles = batch_tiles(b, false);
     for (int j = 0; j < nb && e == cudaSuccess; ++j) e = cudaStreamWaitEvent(b->branch[j], b->fork, 0);
     for (size_t i = 0; i < b->models.size() && e == cudaSuccess; ++i) {
         sgfd_solver *h = b->models[i];
         SourceRec sr = h->sr;
         sr.it_dev = b->step_ctr;
         sr.overlap = 0;
+        const ZGeom g = batch_geom(h, tiles, 0);
         for (int k = 0; k < kGraphSteps && e == cudaSuccess; ++k)
-            e = dispatch_on(h, sr, b->branch[i % nb], k, 0.0f, true, nullptr);
+            e = dispatch_on(h, g, sr, b->branch[i % nb], k, 0.0f, true, nullptr);
     }
     for (int j = 0; j < nb && e == cudaSuccess; ++j) {
         e = cudaEventRecord(b->join[j], b->branch[j]);
@@ -142,6 +152,7 @@ int build_descriptors(sgfd_batch *b) {
     std::vector<ZModel> d(n);
     std::vector<int> first(n + 1, 0);
     b->psame = true;
+    const int64_t tiles = batch_tiles(b, true);
     for (int i = 0; i < n; ++i) {
         const sgfd_solver *h = b->models[i];
         std::memset(static_cast<void *>(&d[i]), 0, sizeof d[i]);
@@ -149,10 +160,10 @@ int build_descriptors(sgfd_batch *b) {
         d[i].m = h->m;
         d[i].ph = h->ph;
         b->psame = b->psame && std::memcmp(&h->ph, &b->models[0]->ph, sizeof h->ph) == 0;
-        d[i].g = h->zg;
+        d[i].g = batch_geom(h, tiles, b->ctas);
         d[i].sr = h->sr;
         d[i].sr.it_dev = nullptr;
-        d[i].items = h->zg.ntx * h->zg.nty * h->zg.nchunks;
+        d[i].items = d[i].g.ntx * d[i].g.nty * d[i].g.nchunks;
         first[i + 1] = first[i] + d[i].items;
     }
     if (!b->pdesc) {
@@ -259,10 +270,10 @@ int sgfd_autotune(sgfd_solver *h, int32_t probe_steps, sgfd_tuning *out) {
         if (r == SGFD_OK && cands[c].kernel == SGFD_KERNEL_ZMARCH)
             r = sgfd_set_tile(h, cands[c].cols, cands[c].rows, cands[c].zchunk);
         if (r) break;
-        cudaError_t e = dispatch_on(h, h->sr, h->stream, 0, 0.0f, false, nullptr);   // warm-up step
+        cudaError_t e = dispatch_on(h, h->zg, h->sr, h->stream, 0, 0.0f, false, nullptr);   // warm-up step
         if (e == cudaSuccess) e = cudaEventRecord(e0, h->stream);
         for (int k = 0; k < probe_steps && e == cudaSuccess; ++k)
-            e = dispatch_on(h, h->sr, h->stream, k, 0.0f, false, nullptr);
+            e = dispatch_on(h, h->zg, h->sr, h->stream, k, 0.0f, false, nullptr);
         if (e == cudaSuccess) e = cudaEventRecord(e1, h->stream);
         if (e == cudaSuccess) e = cudaEventSynchronize(e1);
         float ms = 0.0f;
@@ -396,7 +407,7 @@ int sgfd_batch_run(sgfd_batch *b, int32_t it0, int32_t nsteps) {
     }
     for (; left > 0; --left, ++it)
         for (sgfd_solver *h : b->models)
-            BATCH_CUDA(b, dispatch_on(h, h->sr, b->stream, it, 0.0f, true, nullptr), "batch step launch");
+            BATCH_CUDA(b, dispatch_on(h, h->zg, h->sr, b->stream, it, 0.0f, true, nullptr), "batch step launch");
     BATCH_CUDA(b, cudaEventRecord(b->done, b->stream), "order model streams after the batch");
     for (sgfd_solver *h : b->models)
         BATCH_CUDA(b, cudaStreamWaitEvent(h->stream, b->done, 0), "order model streams after the batch");

@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "solver.h"
+#include "zchunks.h"
 
 using namespace sgfd;
 
@@ -115,14 +116,14 @@ size_t stride16(const sgfd_solver *h) {
     return (size_t)(reinterpret_cast<const char *>(h->hs.f[1]) - reinterpret_cast<const char *>(h->hs.f[0]));
 }
 
-cudaError_t dispatch_on(sgfd_solver *h, const SourceRec &sr, cudaStream_t s, int it, float value,
+cudaError_t dispatch_on(sgfd_solver *h, const ZGeom &g, const SourceRec &sr, cudaStream_t s, int it, float value,
                         bool use_wavelet, cudaEvent_t *ev) {
     const bool h16 = h->storage != SGFD_STORE_F32;
     cudaError_t e = h->kernel == SGFD_KERNEL_ZMARCH
-                        ? (h->zg.pair ? zpair_step(h->m, h->ph, sr, h16 ? &h->hs : nullptr, h->zg, h->vm, h->sm, it,
-                                                   value, use_wavelet, s, ev)
-                           : h16 ? ztwin16_step(h->m, h->ph, sr, h->hs, h->zg, h->tm16, it, value, use_wavelet, s, ev)
-                                 : zmarch_step(h->m, h->ph, sr, h->zg, h->zm, it, value, use_wavelet, s, ev))
+                        ? (g.pair ? zpair_step(h->m, h->ph, sr, h16 ? &h->hs : nullptr, g, h->vm, h->sm, it, value,
+                                              use_wavelet, s, ev)
+                           : h16 ? ztwin16_step(h->m, h->ph, sr, h->hs, g, h->tm16, it, value, use_wavelet, s, ev)
+                                 : zmarch_step(h->m, h->ph, sr, g, h->zm, it, value, use_wavelet, s, ev))
                     : h16 ? half_step(h->m, h->ph, sr, h->hs, it, value, use_wavelet, s, ev)
                         : simple_step(h->m, h->ph, sr, it, value, use_wavelet, s, ev);
     if (e == cudaSuccess && h->strip_n > 0)
@@ -154,6 +155,7 @@ void graph_key(const sgfd_solver *h, GraphKey *k) {
     std::memcpy(static_cast<void *>(&k->zm), &h->zm, sizeof h->zm);
     std::memcpy(static_cast<void *>(&k->tm16), &h->tm16, sizeof h->tm16);
     k->kernel = h->kernel;
+    k->zchunk_req = h->zchunk_req;
     k->audit_every = h->audit_every;
     k->audit_region = h->audit_region;
     k->audit_count = h->audit_count;
@@ -163,6 +165,24 @@ void graph_key(const sgfd_solver *h, GraphKey *k) {
     k->strip_n = h->strip_n;
     k->strip_cells = h->strip_cells;
     k->strip_buf = h->strip_buf;
+}
+
+// nz planes in chunks of zc (a caller's zc may be any).
+static void cut_chunks(ZGeom *g, int nz, int zc) {
+    g->zc = std::max(1, std::min(zc, nz));
+    g->nchunks = (nz + g->zc - 1) / g->zc;
+}
+
+ZGeom batch_geom(const sgfd_solver *h, int64_t tiles, int ctas) {
+    ZGeom g = h->zg;
+    const bool h16 = h->storage != SGFD_STORE_F32;
+    // 16-bit storage on 64 x 8 tiles, whose taps are converted one by one,
+    // gains nothing (8 models of 100^3: 990 us per step as it is, 1133 with 16 planes)
+    if (h->zchunk_req > 0 || (h16 && g.pair)) return g;
+    const int wave = (g.pair || g.cells > 1 ? 2 : 3) * h->sms;   // CTAs the GPU holds at once
+    cut_chunks(&g, h->m.nzc, ctas > 0 ? persistent_chunk(g.zc, tiles, h->m.nzc, ctas)
+                                      : graph_batch_chunk(g.zc, tiles, h->m.nzc, wave, h16));
+    return g;
 }
 
 }  // namespace sgfd
@@ -246,7 +266,7 @@ void set_physics(sgfd_solver *h) {
 }
 
 cudaError_t dispatch_step(sgfd_solver *h, int it, float value, bool use_wavelet, cudaEvent_t *ev) {
-    return dispatch_on(h, h->sr, h->stream, it, value, use_wavelet, ev);
+    return dispatch_on(h, h->zg, h->sr, h->stream, it, value, use_wavelet, ev);
 }
 
 void release_graph(sgfd_solver *h) {
@@ -271,7 +291,7 @@ int capture_graph(sgfd_solver *h) {
     SG_CUDA(h, cudaStreamBeginCapture(h->cap_stream, cudaStreamCaptureModeThreadLocal), "begin capture");
     cudaError_t e = cudaSuccess;
     for (int k = 0; k < kGraphSteps && e == cudaSuccess; ++k)
-        e = dispatch_on(h, sr, h->cap_stream, k, 0.0f, true, nullptr);
+        e = dispatch_on(h, h->zg, sr, h->cap_stream, k, 0.0f, true, nullptr);
     if (e == cudaSuccess) e = launch_counter(h->step_ctr, kGraphSteps, true, h->cap_stream);
     cudaGraph_t g = nullptr;
     const cudaError_t e_end = cudaStreamEndCapture(h->cap_stream, &g);
@@ -300,40 +320,11 @@ int launch_step(sgfd_solver *h, int it, float value, bool use_wavelet) {
     return SGFD_OK;
 }
 
-// z chunking.  A chunk costs about 2.5 planes of start-up (filling the z
-// queues and the first stages), so long chunks waste least; short ones fill
-// the GPU when the grid has few tiles.  One wave is three CTAs on every SM
-// (measured with 32 x 8 tiles, ms per step, FP32):
-//   * every tile fits one wave with chunks of at most 14 planes: the shortest
-//     such chunk (64^3: 2 planes 0.0226, 14 planes 0.0697; 80^3: 5 planes
-//     0.0436, 14 planes 0.0711; 60 x 60 x 400: 13 planes 0.111, 8 0.122;
-//     where one wave needs longer chunks several waves are faster: 120^3
-//     16 planes 0.1261, 8 planes 0.1226);
-//   * fewer than 16 waves of 16-plane chunks: about four waves, 8 to 16
-//     planes (150^3: 8 planes 0.2161, 16 planes 0.2210; 300 x 200 x 100:
-//     12 planes 0.3443, 8 planes 0.3480, 16 planes 0.3497; 200^3 flat from 8
-//     to 16, 0.424 to 0.430);
-//   * larger grids: 16 waves, at most 48 planes (24, 32 and 48 planes within
-//     1 % on the 394^3 grid, 48 planes 2 % faster than 24 on 522^3).
+// The handle's own z chunks (zchunks.h; a chunk the caller set stays).
 void set_zchunks(sgfd_solver *h) {
     ZGeom &g = h->zg;
     const int tiles = g.ntx * g.nty, nz = h->m.nzc;
-    int zc = h->zchunk_req;
-    if (zc <= 0) {
-        const int wave = 3 * h->sms;
-        auto chunk = [&](int waves) {
-            const int n = (waves * wave + tiles - 1) / tiles;
-            return (nz + n - 1) / n;
-        };
-        const int per_tile = wave / tiles;   // chunks of every tile that one wave holds
-        const int single = per_tile > 0 ? (nz + per_tile - 1) / per_tile : nz;
-        if (single <= 14) zc = single;
-        else if (chunk(16) < 16) zc = std::min(16, std::max(8, chunk(4)));
-        else zc = std::min(48, chunk(16));
-    }
-    zc = std::max(1, std::min(zc, nz));
-    g.zc = zc;
-    g.nchunks = (nz + zc - 1) / zc;
+    cut_chunks(&g, nz, h->zchunk_req > 0 ? h->zchunk_req : solo_chunk(tiles, nz, h->sms));
     // launches overlap (step_launch) where their latency shows: the eight
     // launches of a 16-bit step, and grids of at most one wave
     h->sr.overlap = h->storage != SGFD_STORE_F32 || (int64_t)tiles * g.nchunks <= 3 * h->sms;

@@ -25,6 +25,7 @@ struct GraphKey {
     ZMaps zm;
     ZTwin16Maps tm16;
     int kernel;
+    int zchunk_req;      // a batch chooses automatic chunks itself
     int audit_every, audit_region, audit_count;
     double *audit_hist, *audit;
     int strip_w, strip_n;
@@ -124,10 +125,15 @@ int reset_scales(sgfd_solver *h);
 int get_scale_exponents(sgfd_solver *h, int *e);
 int set_scale_exponents(sgfd_solver *h, const int *e);
 
-// Launch one step of h's kernels on stream s with the given receiver /
-// source record (h->sr, or a copy whose it_dev points at a step counter).
-cudaError_t dispatch_on(sgfd_solver *h, const SourceRec &sr, cudaStream_t s, int it, float value,
+// Launch one step of h's kernels on stream s with the given launch geometry
+// (h->zg, or a batch's) and receiver / source record (h->sr, or a copy whose
+// it_dev points at a step counter).
+cudaError_t dispatch_on(sgfd_solver *h, const ZGeom &g, const SourceRec &sr, cudaStream_t s, int it, float value,
                         bool use_wavelet, cudaEvent_t *ev);
+// h's launch geometry as one model of a batch with `tiles` z-march tiles in
+// all: graph replays (ctas 0) or the persistent launch of that many CTAs.
+// Chunks the caller set stay; automatic ones are chosen for the whole batch.
+ZGeom batch_geom(const sgfd_solver *h, int64_t tiles, int ctas);
 // Byte image of everything a captured step passes to h's kernels.
 void graph_key(const sgfd_solver *h, GraphKey *k);
 
