@@ -172,10 +172,13 @@ int build_descriptors(sgfd_batch *b) {
         BATCH_CUDA(b, cudaMalloc(&b->pstatus, sizeof(int)), "batch status");
         BATCH_CUDA(b, cudaMemset(b->pstatus, 0, sizeof(int)), "batch status");
     }
-    BATCH_CUDA(b, cudaMemcpy(b->pdesc, d.data(), (size_t)n * sizeof(ZModel), cudaMemcpyHostToDevice),
+    // a launch still running reads the former descriptors
+    BATCH_CUDA(b, cudaStreamSynchronize(b->stream), "batch descriptors");
+    BATCH_CUDA(b, cudaMemcpyAsync(b->pdesc, d.data(), (size_t)n * sizeof(ZModel), cudaMemcpyHostToDevice, b->stream),
                "batch descriptors");
-    BATCH_CUDA(b, cudaMemcpy(b->pfirst, first.data(), (size_t)(n + 1) * sizeof(int), cudaMemcpyHostToDevice),
-               "batch descriptors");
+    BATCH_CUDA(b, cudaMemcpyAsync(b->pfirst, first.data(), (size_t)(n + 1) * sizeof(int), cudaMemcpyHostToDevice,
+                                  b->stream), "batch descriptors");
+    BATCH_CUDA(b, cudaStreamSynchronize(b->stream), "batch descriptors");
     b->pkeys.resize(n);
     for (int i = 0; i < n; ++i) graph_key(b->models[i], &b->pkeys[i]);
     return SGFD_OK;
