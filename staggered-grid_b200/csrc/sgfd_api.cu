@@ -324,7 +324,8 @@ int launch_step(sgfd_solver *h, int it, float value, bool use_wavelet) {
 void set_zchunks(sgfd_solver *h) {
     ZGeom &g = h->zg;
     const int tiles = g.ntx * g.nty, nz = h->m.nzc;
-    cut_chunks(&g, nz, h->zchunk_req > 0 ? h->zchunk_req : solo_chunk(tiles, nz, h->sms));
+    cut_chunks(&g, nz, h->zchunk_req > 0 ? h->zchunk_req
+                                         : solo_chunk(tiles, nz, h->sms, g.pair, h->storage != SGFD_STORE_F32));
     // launches overlap (step_launch) where their latency shows: the eight
     // launches of a 16-bit step, and grids of at most one wave
     h->sr.overlap = h->storage != SGFD_STORE_F32 || (int64_t)tiles * g.nchunks <= 3 * h->sms;

@@ -29,15 +29,26 @@ inline int chunk_of(int nz, int64_t chunks) {   // planes of each of `chunks` eq
 //     to 16, 0.424 to 0.430);
 //   * larger grids: 16 waves, at most 48 planes (24, 32 and 48 planes within
 //     1 % on the 394^3 grid, 48 planes 2 % faster than 24 on 522^3).
-inline int solo_chunk(int tiles, int nz, int sms) {
+// The 64 x 8 tiles (pair) run two CTAs on an SM, so their one wave is that
+// (ms per step, FP32 then FP16: 90^3 4 planes 0.0997, 0.124, 6 planes 0.0815,
+// 0.0991; 130^3 FP16 9 planes 0.276, 14 planes 0.243); the other lines count
+// CTAs and stay.  With 16-bit storage (half) each tap of theirs is converted
+// as it is read and a chunk's start-up is dearer: 16 planes where such chunks
+// make two waves of a grid of at least 64 planes (180^3 8 planes 0.687, 16
+// planes 0.650; 157 x 333 x 91 8 planes 0.612, evened out to 14 0.583; below
+// two waves 140^3 8 planes 0.392, 15 0.453, and on flat grids 1000 x 300 x 30
+// 8 planes 0.645, 10 0.697), evened out if the last would hold one or two.
+inline int solo_chunk(int tiles, int nz, int sms, bool pair = false, bool half = false) {
     const int wave = 3 * sms;
     auto waves = [&](int w) { return chunk_of(nz, ((int64_t)w * wave + tiles - 1) / tiles); };
-    const int per_tile = wave / tiles;   // chunks of every tile that one wave holds
+    const int per_tile = (pair ? 2 : 3) * sms / tiles;   // chunks of every tile that one wave holds
     const int single = per_tile > 0 ? chunk_of(nz, per_tile) : nz;
+    const int n16 = (nz + 15) / 16;
     int zc;
     if (single <= 14) zc = single;
-    else if (waves(16) < 16) zc = std::min(16, std::max(8, waves(4)));
-    else zc = std::min(48, waves(16));
+    else if (waves(16) >= 16) zc = std::min(48, waves(16));
+    else if (pair && half && nz >= 64 && (int64_t)tiles * n16 >= 4 * sms) zc = (nz - 1) % 16 < 2 ? chunk_of(nz, n16) : 16;
+    else zc = std::min(16, std::max(8, waves(4)));
     return std::max(1, std::min(zc, nz));
 }
 

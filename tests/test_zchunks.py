@@ -22,6 +22,16 @@ int main() {
       std::printf("solo %d x %d: %d, not %d\n", c[0], c[1], solo_chunk(c[0], c[1], kSms), c[2]);
       return 1;
     }
+  // 64 x 8 tiles (FP32, 16 bits): one wave of two CTAs per SM, then as above, or chunks of 16 planes
+  const int pairs[][4] = {{20, 80, 6, 6}, {30, 120, 14, 14}, {51, 130, 8, 8}, {66, 170, 8, 16},
+                          {123, 81, 8, 14}, {72, 190, 8, 16}, {592, 20, 8, 8}, {592, 46, 16, 16},
+                          {144, 256, 16, 16}, {9, 390, 13, 13}};
+  for (auto &c : pairs)
+    for (int half = 0; half < 2; ++half)
+      if (solo_chunk(c[0], c[1], kSms, true, half) != c[2 + half]) {
+        std::printf("64 x 8, %d x %d, half %d: %d\n", c[0], c[1], half, solo_chunk(c[0], c[1], kSms, true, half));
+        return 1;
+      }
   for (int edge = 20; edge <= 400; ++edge) {
     const int nz = edge - 10, t = tiles_of(nz), own = solo_chunk(t, nz, kSms);
     for (int n : {1, 2, 3, 4, 8, 12, 16, 32, 64, 200}) {
