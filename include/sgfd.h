@@ -315,7 +315,9 @@ int sgfd_step_phase(sgfd_solver *h, int32_t it, float source_value, int32_t phas
  * simple ones): they read no frame plane, so they may run while the halos are
  * in flight.  SGFD_PART_OUTER updates the rest, after the unpack.  Run INNER
  * before OUTER (the simple kernels inject the source with INNER and record
- * the receivers with OUTER); INNER | OUTER is sgfd_step_phase. */
+ * the receivers with OUTER); INNER | OUTER is sgfd_step_phase.  A z-marching
+ * handle whose inner part is too small to hide an exchange (less than one wave
+ * of CTAs) does all of it in OUTER: INNER then launches nothing. */
 #define SGFD_PART_INNER 1
 #define SGFD_PART_OUTER 2
 int sgfd_step_phase_part(sgfd_solver *h, int32_t it, float source_value, int32_t phase, int32_t parts);

@@ -780,6 +780,18 @@ int sgfd_step_phase_part(sgfd_solver *h, int32_t it, float source_value, int32_t
     if (h->strip_n > 0 || h->audit_every > 0)
         return fail(h, SGFD_ERR_UNSUPPORTED, "half steps run neither a learned strip nor a per-step audit");
     const int phases = phase == SGFD_PHASE_VELOCITY ? 1 : 2;
+    if (h->kernel == SGFD_KERNEL_ZMARCH && parts != (SGFD_PART_INNER | SGFD_PART_OUTER)) {
+        // An inner part of less than one wave hides less of an exchange than
+        // the two launches more that it costs: it runs with the outer part,
+        // in one launch (64^3 in 4 slabs on one GPU 359 us per step in parts,
+        // 318 like this; 100^3 in 2 163 and 118; 200^3 in 4 514 and 478).
+        int r[3][2];
+        part_ranges(h->m.nzc, h->zg.zc, h->zg.nchunks, kPartInner, r);
+        if ((int64_t)h->zg.ntx * h->zg.nty * (r[0][1] - r[0][0]) < 3 * h->sms) {
+            if (parts == SGFD_PART_INNER) return SGFD_OK;
+            parts = SGFD_PART_INNER | SGFD_PART_OUTER;
+        }
+    }
     SourceRec sr = h->sr;
     sr.overlap = 0;   // the slabs of a model share the GPU
     const cudaError_t e =
