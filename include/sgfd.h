@@ -348,8 +348,9 @@ int sgfd_autotune(sgfd_solver *h, int32_t probe_steps, sgfd_tuning *out);
  * one device) together: one CUDA graph per 16 steps holds every model's
  * kernels in parallel branches, so small models fill the GPU side by side.
  * Each model keeps its own medium, source, receivers and wavelet (set through
- * its handle before the run); the batch only launches.  The models stay
- * owned by the caller and must outlive the batch. */
+ * its handle before the run); the batch only launches.  Automatic z chunks are
+ * chosen for the batch as a whole (sgfd_get_tile keeps saying the model's own).
+ * The models stay owned by the caller and must outlive the batch. */
 typedef struct sgfd_batch sgfd_batch;
 int sgfd_batch_create(sgfd_solver *const *models, int32_t n, sgfd_batch **out);
 void sgfd_batch_destroy(sgfd_batch *b);

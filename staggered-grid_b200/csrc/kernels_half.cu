@@ -378,15 +378,17 @@ cudaError_t step16(const Model &m, const Physics &ph, const SourceRec &sr, const
 template <int ST>
 cudaError_t phases16(const Model &m, const Physics &ph, const SourceRec &sr, const HalfState &hs, int it,
                      float src_value, bool use_wavelet, cudaStream_t s, int phase) {
+    const bool overlap = sr.overlap != 0;
     if (phase == 0) {
-        if (sr.src >= 0) step_launch(k_inject16<ST>, 1, 32, 0, s, sr.overlap != 0, m, ph, sr, hs, it, src_value, use_wavelet ? 1 : 0);
+        if (sr.src >= 0)
+            step_launch(k_inject16<ST>, 1, 32, 0, s, overlap, m, ph, sr, hs, it, src_value, use_wavelet ? 1 : 0);
     } else if (phase == 1) {
-        if (sr.nrec > 0) step_launch(k_record16<ST>, (sr.nrec + 127) / 128, 128, 0, s, sr.overlap != 0, m, sr, hs, it, 1);
+        if (sr.nrec > 0) step_launch(k_record16<ST>, (sr.nrec + 127) / 128, 128, 0, s, overlap, m, sr, hs, it, 1);
     } else {
-        if (sr.nrec > 0) step_launch(k_record16<ST>, (sr.nrec + 127) / 128, 128, 0, s, sr.overlap != 0, m, sr, hs, it, 0);
-        step_launch(k_rescale_choose, 1, 32, 0, s, sr.overlap != 0, sr, hs, it);
-        step_launch(k_rescale_apply<ST>, 1184, 256, 0, s, sr.overlap != 0, m, sr, hs, it, m.plane * m.nz);
-        step_launch(k_rescale_commit, 1, 32, 0, s, sr.overlap != 0, sr, hs, it);
+        if (sr.nrec > 0) step_launch(k_record16<ST>, (sr.nrec + 127) / 128, 128, 0, s, overlap, m, sr, hs, it, 0);
+        step_launch(k_rescale_choose, 1, 32, 0, s, overlap, sr, hs, it);
+        step_launch(k_rescale_apply<ST>, 1184, 256, 0, s, overlap, m, sr, hs, it, m.plane * m.nz);
+        step_launch(k_rescale_commit, 1, 32, 0, s, overlap, sr, hs, it);
     }
     return cudaGetLastError();
 }
@@ -395,8 +397,9 @@ cudaError_t phases16(const Model &m, const Physics &ph, const SourceRec &sr, con
 
 cudaError_t half_phase(const Model &m, const Physics &ph, const SourceRec &sr, const HalfState &hs, int it,
                        float src_value, bool use_wavelet, cudaStream_t s, int phase) {
-    return hs.storage == SGFD_STORE_BF16 ? phases16<SGFD_STORE_BF16>(m, ph, sr, hs, it, src_value, use_wavelet, s, phase)
-                                         : phases16<SGFD_STORE_F16>(m, ph, sr, hs, it, src_value, use_wavelet, s, phase);
+    return hs.storage == SGFD_STORE_BF16
+               ? phases16<SGFD_STORE_BF16>(m, ph, sr, hs, it, src_value, use_wavelet, s, phase)
+               : phases16<SGFD_STORE_F16>(m, ph, sr, hs, it, src_value, use_wavelet, s, phase);
 }
 
 cudaError_t half_step(const Model &m, const Physics &ph, const SourceRec &sr, const HalfState &hs, int it,

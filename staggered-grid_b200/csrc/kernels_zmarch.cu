@@ -271,8 +271,8 @@ __device__ __forceinline__ bool vel_item(const ZMaps &mp, const Model &m, const 
         const int kz = bandz(m, gz);
         const bool plane_pml = GEN && (t.xy_pml || kz != 0);
 
-
-        // PML cells: splits and damping speed, loaded before the stage wait so that their latency overlaps the wait and the stencil
+        // PML cells: splits and damping speed, loaded before the stage wait so
+        // that their latency overlaps the wait and the stencil
         float opre[CELLS][9], vpre[CELLS];
         if (plane_pml) {
 #pragma unroll
@@ -548,8 +548,8 @@ __device__ __forceinline__ bool str_item(const ZMaps &mp, const Model &m, const 
         pcol[c] = pml_column(m, min(t.cx0 + lx, m.nxc - 1), min(t.cy0 + lyc[c], m.nyc - 1));
     }
 
-    // z queues, 11 deep, planes in pairs as in the velocity update: before the
-    // first plane of a pair at z, qx and qy (vx, vy) hold z-4..z+4 and qz (vz)
+    // z queues, 11 deep, moved by two after each pair of planes (the velocity
+    // update's move by one): before the first plane of a pair at z, qx and qy (vx, vy) hold z-4..z+4 and qz (vz)
     // z-5..z+3 in slots 0..8
     float qx[CELLS][11], qy[CELLS][11], qz[CELLS][11];
     const int gz0 = t.zs + kHalo;
@@ -881,7 +881,8 @@ __device__ __noinline__ bool str_item_call(const ZMaps &mp, const Model &m, cons
 // do; the updates, inlined, then take their constants from the constant bank
 // as single launches do.  Otherwise each model's physics is copied to shared
 // memory, read there in every plane's inner loops (12 models of 146^3 to
-// 306^3, 16 steps: 135.5 ms that way, 126.7 ms with SAME).
+// 306^3, 16 steps: 127.7 ms with SAME, 136.3 ms with one model's damping
+// constant changed).
 // Two CTAs per SM: with the 80 registers a thread of three CTAs both updates
 // spill beside the loop's own state (SAME 145.8 ms, called 171.4 ms).
 template <bool FAST, bool SAME>

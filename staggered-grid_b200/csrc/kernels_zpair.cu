@@ -212,12 +212,6 @@ __device__ __forceinline__ void window(const float *row, float (&w)[12]) {
     }
 }
 __device__ __forceinline__ float lane_of(float2 v, int c) { return c ? v.y : v.x; }
-// Element k of a six-value register array without indexing it at run time
-// (which would move the array to local memory).
-template <class T>
-__device__ __forceinline__ T pick6(const T (&a)[6], int k) {
-    return k == 0 ? a[0] : k == 1 ? a[1] : k == 2 ? a[2] : k == 3 ? a[3] : k == 4 ? a[4] : a[5];
-}
 
 __device__ __forceinline__ void st2(float *p, float2 v, bool both) {
     if (both) *reinterpret_cast<float2 *>(p) = v;

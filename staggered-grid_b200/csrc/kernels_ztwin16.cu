@@ -56,7 +56,8 @@ using namespace zdev;
 
 constexpr int TX = kZTileX, TY = 8, NT = 256;
 constexpr int W48 = 48, W32 = 32, W36 = 36;
-constexpr int N48 = W48 * TY, N48Y = W48 * (TY + 10), N32Y = W32 * (TY + 10), N32 = W32 * TY;   // values of a box's plane
+// values of a box's plane
+constexpr int N48 = W48 * TY, N48Y = W48 * (TY + 10), N32Y = W32 * (TY + 10), N32 = W32 * TY;
 
 constexpr int al128(int b) { return (b + 127) / 128 * 128; }
 
@@ -546,7 +547,8 @@ k_stress_ztwin16(const __grid_constant__ ZTwin16Maps mp, const __grid_constant__
             // shear stresses last: their differences wait for no copy
             float2 a, b;
             dZ2(a, b);
-            const float2 sxy = __fadd2_rn(by_cell2<FAST>(ph, 1, fwd2<W48>(cY, vx)), by_cell2<FAST>(ph, 0, fwd2<1>(cX, vy)));
+            const float2 sxy =
+                __fadd2_rn(by_cell2<FAST>(ph, 1, fwd2<W48>(cY, vx)), by_cell2<FAST>(ph, 0, fwd2<1>(cX, vy)));
             const float2 sxz = __fadd2_rn(make_float2(a.x, b.x), by_cell2<FAST>(ph, 0, fwd2<1>(cX, vz)));
             const float2 syz = __fadd2_rn(make_float2(a.y, b.y), by_cell2<FAST>(ph, 1, fwd2<W48>(cY, vz)));
             const float2 dXx = by_cell2<FAST>(ph, 0, bwd2<1>(cX, vx)), dYy = by_cell2<FAST>(ph, 1, bwd2<W48>(cY, vy)),
@@ -671,7 +673,8 @@ void launch(const Model &m, const Physics &ph, const SourceRec &sr, const HalfSt
     const dim3 grid(g.ntx * g.nty, g.nchunks);
     half_phase(m, ph, sr, hs, it, src_value, uw, s, 0);
     if (ev) cudaEventRecord(ev[0], s);
-    step_launch(k_velocity_ztwin16<FAST, ST>, grid, NT, smem_bytes<VelH>(), s, sr.overlap != 0, tm, m, ph, g, sr, hs, it);
+    step_launch(k_velocity_ztwin16<FAST, ST>, grid, NT, smem_bytes<VelH>(), s, sr.overlap != 0, tm, m, ph, g, sr, hs,
+                it);
     if (ev) cudaEventRecord(ev[1], s);
     half_phase(m, ph, sr, hs, it, src_value, uw, s, 1);
     if (ev) cudaEventRecord(ev[2], s);

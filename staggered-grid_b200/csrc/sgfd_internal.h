@@ -118,12 +118,15 @@ struct SourceRec {
 };
 
 #ifdef __CUDACC__
-// The kernels of a step call this first, every thread of them: wait until the
-// launch before has completed and its stores are visible, then let the next
-// launch's blocks be scheduled as this one's drain.  A kernel that returned
-// without waiting would complete before its predecessor and let its successor
-// run ahead of both.  Without the launch attribute of step_launch both
-// instructions do nothing.
+// The kernels that step_launch launches (the z-march updates on 32-column
+// tiles and the 16-bit source, receiver and rescale kernels) call this first,
+// every thread of them: wait until the launch before has completed and its
+// stores are visible, then let the next launch's blocks be scheduled as this
+// one's drain.  A kernel that returned without waiting would complete before
+// its predecessor and let its successor run ahead of both.  Launched without
+// the attribute of step_launch, a kernel has nothing to wait for; the release
+// holds all the same, and reaches a next launch that carries the attribute
+// (one of ours, or a caller's own on the same stream, which has to wait too).
 __device__ __forceinline__ void step_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -132,7 +135,9 @@ __device__ __forceinline__ void step_wait() {
 // programmatic-serialisation attribute, so that its blocks become resident and
 // set themselves up while the last blocks of the launch before still run.
 // For one stream of launches only: resident blocks that wait would take room
-// from another stream's kernels (batches, z-slabs).  Measured, us per step
+// from another stream's kernels (graph replays of a batch and z-slabs keep
+// plain launches; the steps a batch has left after its replays run on one
+// stream).  Measured, us per step
 // without and with it: FP32 launched step by step 40^3 16.5 and 14.1, 64^3
 // 26.5 and 22.4, 100^3 71.1 and 69.8, 150^3 215 and 216 (more than one wave:
 // off); FP32 graph replays 64^3 22.3 and 21.8, 100^3 67.5 and 68.8, 150^3 210

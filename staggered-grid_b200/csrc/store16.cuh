@@ -26,16 +26,10 @@ struct H16 {
     }
 };
 
-// Largest |v| of the warp's active lanes into field g's running maximum (the
-// rescale steps of 16-bit storage, as kernels_half.cu notes them).
-__device__ __forceinline__ void note_max16(const HalfState &hs, int g, float v) {
-    const unsigned mask = __activemask();
-    const unsigned bits = __reduce_max_sync(mask, __float_as_uint(fabsf(v)));
-    if ((threadIdx.x & 31) == __ffs(mask) - 1) atomicMax(hs.amax + g, bits);
-}
-
-// The same into a CTA's shared running maxima (smax[g], unsigned float
-// bits); the CTA adds them to the global ones once (flush_max16).
+// Largest |v| (as unsigned float bits) of the warp's active lanes into field
+// g's running maximum of the CTA, in shared memory (the rescale steps of 16-bit
+// storage, as kernels_half.cu notes them); the CTA adds its maxima to the
+// global ones once (flush_max16).
 __device__ __forceinline__ void note_bits16s(unsigned *smax, int g, unsigned v) {
     const unsigned mask = __activemask();
     const unsigned bits = __reduce_max_sync(mask, v);

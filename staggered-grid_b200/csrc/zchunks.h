@@ -13,9 +13,10 @@ inline int chunk_of(int nz, int64_t chunks) {   // planes of each of `chunks` eq
 }
 
 // A model on its own, `tiles` tiles of nz planes on a GPU of `sms` SMs.  A
-// chunk starts by filling the z queues and the first stages: about 2.5 planes
-// of work in a lone short wave, 0.3 planes on a filled GPU (150^3, 200^3, 300 x
-// 200 x 100 below).  Long chunks waste least of it; short ones fill the GPU
+// chunk starts by filling the z queues and the first stages: two to three
+// planes' time in a lone short wave (64^3, launches included), 0.3 planes' on
+// a filled GPU (150^3: 196.6 us per step with 2-plane chunks, 182.1 with 4,
+// 175.6 with 8).  Long chunks waste least of it; short ones fill the GPU
 // when the grid has few tiles.  One wave is three CTAs on every SM (measured
 // with 32 x 8 tiles, ms per step, FP32):
 //   * every tile fits one wave with chunks of at most 14 planes: the shortest
@@ -47,7 +48,8 @@ inline int solo_chunk(int tiles, int nz, int sms, bool pair = false, bool half =
     int zc;
     if (single <= 14) zc = single;
     else if (waves(16) >= 16) zc = std::min(48, waves(16));
-    else if (pair && half && nz >= 64 && (int64_t)tiles * n16 >= 4 * sms) zc = (nz - 1) % 16 < 2 ? chunk_of(nz, n16) : 16;
+    else if (pair && half && nz >= 64 && (int64_t)tiles * n16 >= 4 * sms)
+        zc = (nz - 1) % 16 < 2 ? chunk_of(nz, n16) : 16;
     else zc = std::min(16, std::max(8, waves(4)));
     return std::max(1, std::min(zc, nz));
 }

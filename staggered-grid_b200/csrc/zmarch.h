@@ -62,7 +62,7 @@ struct ZGeom {
     int ntx, nty;
     int zc, nchunks;
     int c0;                 // first z chunk of this launch (blockIdx.y = chunk - c0); 0 for a whole half step
-    const int *rec_off;     // ntx*nty + 1 offsets into rec_list / rec_idx
+    const int *rec_off;     // ntx*nty + 1 offsets into rec_list / rec_col
     const int4 *rec_list;   // GRID x, y, z, component
     const int2 *rec_col;    // trace column; end of the entries on the same tile and plane
     int *err;               // device error flag (1: a bounded wait gave up)

@@ -1,7 +1,8 @@
 // zmarch_dev.cuh — device helpers shared by the z-marching kernel families
-// (kernels_zmarch.cu, kernels_zpair.cu): mbarrier waits with an iteration
-// cap, TMA tiled loads (no multicast), shared-memory alignment and the
-// bounded grid barrier of the persistent batch kernel.
+// (kernels_zmarch.cu, kernels_ztwin16.cu, kernels_zpair.cu): mbarrier waits
+// with an iteration cap, TMA tiled loads (no multicast), split-row prefetch,
+// receiver recording, shared-memory alignment and the bounded grid barrier of
+// the persistent batch kernel.
 #pragma once
 
 #include <cuda.h>
@@ -69,18 +70,16 @@ __device__ __forceinline__ void l2_prefetch(const void *p, uint32_t bytes) {
 // Warp-wide, all lanes: for the lanes whose cell is a PML cell (pml) with
 // compact index idx, bring rows [k0, k1) of every split block those cells
 // lie in into L2 (one bulk prefetch per block, from lanes 0, 1, ...).
-// Returns whether any lane's cell is a PML cell.
 template <class T>
-__device__ __forceinline__ bool prefetch_split_rows(const T *split, bool pml, uint32_t idx, int k0, int k1,
+__device__ __forceinline__ void prefetch_split_rows(const T *split, bool pml, uint32_t idx, int k0, int k1,
                                                     int lane) {
     const uint32_t lo = __reduce_min_sync(0xffffffffu, pml ? idx : 0xffffffffu);
-    if (lo == 0xffffffffu) return false;
+    if (lo == 0xffffffffu) return;
     const uint32_t hi = __reduce_max_sync(0xffffffffu, pml ? idx : 0u);
     const uint32_t b0 = lo / kSplitBlock;
     if ((uint32_t)lane <= hi / kSplitBlock - b0)
         l2_prefetch(split + (size_t)(b0 + lane) * (kNumSplit * kSplitBlock) + k0 * kSplitBlock,
                     (uint32_t)((k1 - k0) * kSplitBlock * sizeof(T)));
-    return true;
 }
 
 // Wait (bounded) for the stages still in flight before an early exit:
