@@ -247,7 +247,10 @@ float sgfd_ricker_t0(float f0, float dt, float t0, int32_t it);
 int sgfd_profile(sgfd_solver *h, int32_t it0, int32_t nsteps, float *ms_velocity, float *ms_stress);
 
 /* z-marching kernels: planes per z chunk (0 = automatic).  Larger chunks
- * re-read fewer warm-up planes; smaller ones give more CTAs to balance. */
+ * re-read fewer warm-up planes; smaller ones give more CTAs to balance.  The
+ * automatic chunk lets this model fill the GPU alone; a batch chooses it for
+ * all its models.  Many small handles that a program runs at once on streams of
+ * their own do better in a batch, or with chunks of 8 planes or more set here. */
 int sgfd_set_zchunk(sgfd_solver *h, int32_t planes);
 
 /* Switch the kernel family of an existing handle (SGFD_KERNEL_AUTO means
